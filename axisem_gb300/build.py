@@ -2,7 +2,7 @@
 
     python -c "import axisem_gb300.build as b; b.build()"
 
-compiles ``csrc/axg_api.cu`` and ``csrc/axg_plan.cpp`` for sm_103a into
+compiles ``csrc/axg_api.cu``, ``csrc/axg_stream_*.cu`` and ``csrc/axg_plan.cpp`` for sm_103a into
 ``axisem_gb300/_build/libaxisem_gb300.so``.  The translation units are
 compiled in parallel; a rebuild happens only when a source is newer than the
 library.
@@ -26,7 +26,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", str(ROO
           "-I", str(CSRC)]
 CUDA_FLAGS = ARCH + ["-ftz=true", "-prec-div=true", "-prec-sqrt=true", "--expt-relaxed-constexpr"]
 
-SOURCES = ["axg_api.cu", "axg_plan.cpp"]
+SOURCES = ["axg_api.cu", "axg_stream_mono.cu", "axg_stream_di.cu", "axg_stream_quad.cu", "axg_plan.cpp"]
 
 
 def nvcc() -> str:

@@ -1,11 +1,12 @@
 // axg_api.cu -- the C-ABI of include/axisem_gb300.h.
 //
-// axg_create validates the descriptor, plans the patch colouring of the
-// solid and fluid domains (axg_plan.cpp), packs the per-element data in
-// launch order (one contiguous block of metric terms per element), builds the
-// solid-fluid coupling tables and copies everything to HBM.  axg_run advances
-// the Newmark loop of SOLVER/time_evol_wave.F90:353-500 with the kernels of
-// axg_kernels.cuh, captured in CUDA graphs of `steps_per_graph` steps.
+// axg_create validates the descriptor, plans patches of the solid and fluid
+// domains (axg_plan.cpp) and the streamed step's order and point numbering
+// from them, packs the per-element data in groups of six (axg_stream.cuh),
+// builds the solid-fluid coupling tables and copies everything to HBM.
+// axg_run advances the Newmark loop of SOLVER/time_evol_wave.F90:353-500 with
+// the kernels of axg_stream.cuh, captured in CUDA graphs of `steps_per_graph`
+// steps.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -17,13 +18,16 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <thread>
 #include <utility>
 #include <string>
+#include <system_error>
 #include <tuple>
 #include <vector>
 
 #include "axg_kernels.cuh"
 #include "axg_plan.h"
+#include "axg_stream_host.h"
 #include "axisem_gb300.h"
 
 using namespace axg;
@@ -64,22 +68,40 @@ struct DevBuf {
   size_t n = 0;
 };
 
+// one domain of the step on the device (axg_stream.cuh)
 struct DomainDev {
-  PatchMeta *meta = nullptr;
-  uint32_t *pts = nullptr;
-  int32_t *elinfo = nullptr;
-  // the fluid's two passes: element points (launch order), the CSR of each
-  // point's copies (flags in start), the per-copy contributions (per solve)
-  int32_t *gidx = nullptr, *start = nullptr, *ent = nullptr;
-  float *fel = nullptr;
-  float *metric = nullptr;
+  float *blocks = nullptr, *tails = nullptr;
+  int32_t *elinfo = nullptr;      // per slot (the fluid's per solve: source slots)
+  int32_t *start0 = nullptr;      // the mesh's CSR start words (no source flags)
+  int32_t *start = nullptr, *ent = nullptr;  // start: this solve's (solid) or the mesh's (fluid)
+  float *fel = nullptr;           // per solve
   float *m0 = nullptr;
-  float *fsmask = nullptr;
+  float *fsmask = nullptr;        // fluid: per slot 25
   float *srcfl = nullptr;
+  PatchInfo *patches = nullptr;   // patched solid
+  GroupMeta *groups = nullptr;
+  int32_t *def = nullptr;
   // per global point: bit c set where the pole's axis mask zeroes component
   // c (points on the axis), or null
   uint8_t *axmask = nullptr;
-  int64_t n_m0 = 0;
+  int64_t n_m0 = 0, n_ent = 0, n_fel = 0;
+};
+
+// Order of a domain for the step: element slots, groups, the internal point
+// numbering, and for a patched solid its patches.  A patch's own points (held
+// by it alone, not coupled) are consecutive; the deferred points come after
+// all own points (n_own of them, 0 in a scattered domain, whose points are all
+// left to the point pass).
+struct StreamOrder {
+  bool patched = false;
+  std::vector<int32_t> elem_order;              // slot -> element
+  std::vector<int32_t> new_of_old, old_of_new;  // point numbering
+  std::vector<GroupMeta> groups;
+  std::vector<int32_t> group_of_slot;
+  int64_t n_own = 0;
+  std::vector<PatchInfo> patches;
+  std::vector<int32_t> def;                     // deferred points, patch by patch (internal numbers)
+  const GroupMeta &group(int64_t slot) const { return groups[group_of_slot[slot]]; }
 };
 
 // Device buffers of a mesh (element blocks, plans, masses, coupling tables,
@@ -107,11 +129,12 @@ struct axg_handle {
   int32_t niter = 0, seis_it = 1, num_rec = 0, nseismo = 0;
   bool absorbing = false;
   double dt = 0, magnitude = 0;
-  // igloc in the plans' internal point numbering (DomainPlan::new_of_old):
+  // igloc in the internal point numbering (StreamOrder::new_of_old):
   // every per-point table and device array of the handle uses it
   std::vector<int32_t> igloc_s, igloc_f, rec_gidx;
   std::vector<uint8_t> pre_s, pre_f;
-  DomainPlan ps, pf;
+  DomainPlan ps, pf;     // the patches (the streamed step takes its order from them)
+  StreamOrder os, of;
   int patch_elems = 0, growth = -1;  // requested patch shape (0 / -1: tuned)
   int steps_per_graph = 16;
   // device
@@ -123,8 +146,8 @@ struct axg_handle {
   DomainDev ds, df;
   float *su[3] = {}, *sv[3] = {}, *sa[3] = {}, *sf[3] = {};
   std::vector<int32_t> ielsrc;  // the source elements (0-based, solid or fluid as fluid_src says)
-  // The plain Newmark step's predicted displacement (and chi): the last
-  // writers store it into the buffer of the old displacement, and the step's
+  // The Newmark step's predicted displacement (and chi): the point pass
+  // stores it into the buffer of the old displacement, and the step's
   // prediction becomes the new displacement, so the two buffers trade roles
   // (su <-> sup, fu <-> fup) after every such step; `parity` counts the
   // trades modulo 2 (step graphs are captured per parity).
@@ -138,6 +161,7 @@ struct axg_handle {
   float *stf = nullptr, *rec = nullptr;
   int32_t *iter = nullptr, *blowup = nullptr, *rec_gidx_d = nullptr;
   int32_t *src_gidx_d = nullptr;
+  std::vector<int32_t> src_patches;  // patches that own source points (at most 8: one per source element)
   float *src_val_d = nullptr;
   int32_t n_src = 0;
   // gvec I/O in the reference's numbering (made on first use): the solid
@@ -152,11 +176,11 @@ struct axg_handle {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t ev_done = nullptr;  // end of the work axg_run_async queued
   bool pending = false;
-  int num_sms = 1, solid_ctas = 1;
-  int32_t *errw = nullptr;
+  int num_sms = 1;
+  int elem_ctas_force = 1, elem_ctas_step = 1;  // resident CTAs per SM of the element pass
+  int32_t *errw = nullptr, *iter_p = nullptr;
   std::string err = "no error";
   int64_t kernels_per_step = 0, kernels_per_force = 0;
-  int solid_ctas_step = 1;
   // time scheme: 0 Newmark (newmark2), else a symplectic scheme of nstages stages
   int scheme = 0, nstages = 0;
   std::vector<double> sym_cd, sym_cv;  // coefd(1:nstages+1) deltat, coefv(1:nstages) deltat
@@ -164,15 +188,17 @@ struct axg_handle {
   // compensated (Kahan) time integration
   bool kahan = false;
   float *cu_s[3] = {}, *cv_s[3] = {}, *cu_f = nullptr, *cv_f = nullptr;
+  float *cup_s[3] = {}, *cup_f = nullptr;  // after the next step's prediction (scratch of the loop)
   // coarse-grained attenuation
-  bool anel = false;       // coarse-grained (cg4) attenuation, fused into the solid kernel
+  bool anel = false;       // coarse-grained (cg4) attenuation, fused into the element pass
   bool anel_full = false;  // attenuation at every GLL point (anel_full_kernel)
   float *fx = nullptr;     // ... its per-slot force terms for the next step
   int nsls = 0;
-  AnelArgs an{};
+  AnelArgs an{};           // at every GLL point
+  CgArgs cg{};             // cg4
   std::vector<int32_t> slot_of_elem_s;  // solid element -> launch slot
-  int32_t *sym_gidx = nullptr;           // symplectic + attenuation: each launch slot's points
-  uint8_t *sym_axial = nullptr;          // and axis flag
+  int32_t *slot_gidx = nullptr;          // attenuation at every GLL point: each slot's points
+  uint8_t *slot_axial = nullptr;         // and axis flag
   // kernel wavefield dumps (axg_set_wavefield_dump)
   std::vector<uint8_t> axial_s, axial_f;  // per element (reference order): on the axis
   struct Dump {
@@ -399,197 +425,320 @@ std::vector<T> per_point(const T *elem, const std::vector<int32_t> &igloc, int64
   return out;
 }
 
-// The fluid's arrays for its two passes.  mesh_part (mesh pool): the metric
-// blocks, axial vectors and free-surface mask per element slot (launch
-// order), the slots' global points, and per point the CSR of its copies with
-// its flags (a coupling pre-pass partial sum; on the axis); always (this
-// solve): the element info words (source slot), the fluid source terms and
-// the per-copy contribution buffer.
-int build_fluid_passes(axg_handle *h, const axg_mesh_desc *d, const std::vector<int32_t> &order, DomainDev &dd,
-                       bool mesh_part, const std::vector<float> &metric, const std::vector<int32_t> &elinfo,
-                       const std::vector<float> &m0, const std::vector<float> &fsmask, int nax, const int32_t *axl) {
-  const int64_t nel = (int64_t)order.size(), nglob = h->nglob_f, nch = fl_chunks(nel);
-  int rc;
-  if (mesh_part) {
-    if (nch * 25 * kFlChunk >= (int64_t)INT32_MAX) return fail(h, AXG_ERR_BAD_DESC, "fluid mesh too large");
-    std::vector<int32_t> gidx((size_t)nch * 25 * kFlChunk, 0), start(nglob + 1, 0), ent((size_t)25 * nel);
-    for (int64_t s = 0; s < nel; ++s) {
-      const int64_t e = order[s];
-      for (int k = 0; k < 25; ++k) {
-        const int32_t g = h->igloc_f[25 * e + k] - 1;  // internal numbering
-        gidx[fl_at(s, k, 25)] = g;
-        start[g + 1]++;
-      }
-    }
-    for (int64_t g = 0; g < nglob; ++g) start[g + 1] += start[g];
-    if (start[nglob] >= (int64_t)kFlStartMask) return fail(h, AXG_ERR_BAD_DESC, "fluid mesh too large");
-    {
-      // copies in slot order: each point's contributions are summed in the
-      // order of its elements' slots
-      std::vector<int32_t> fill(start.begin(), start.end() - 1);
-      for (int64_t s = 0; s < nel; ++s)
-        for (int k = 0; k < 25; ++k) {
-          const int64_t c = fl_at(s, k, 25);
-          ent[fill[gidx[c]]++] = (int32_t)c;
-        }
-    }
-    // flags: the coupling pre-pass's receiving points, the points on the axis
-    for (size_t g = 0; g < h->pre_f.size(); ++g)
-      if (h->pre_f[g]) start[h->pf.new_of_old[g]] |= (int32_t)kFlPartial;
-    for (int k = 0; k < nax; ++k)
-      for (int jj = 0; jj < 5; ++jj) start[h->igloc_f[25 * (int64_t)(axl[k] - 1) + 5 * jj] - 1] |= (int32_t)kFlAxis;
-    // apply_axis_mask_scal (non-monopole sources) zeroes chi on the axis
-    std::vector<uint8_t> axmask;
-    if (d->src_type != AXG_MONOPOLE && nax > 0) {
-      axmask.assign(nglob, 0);
-      for (int64_t g = 0; g < nglob; ++g) axmask[g] = (start[g] & (int32_t)kFlAxis) ? 1 : 0;
-    }
-    h->in_mesh = true;
-    rc = upload(h, &dd.metric, metric);
-    if (!rc && !axmask.empty()) rc = upload(h, &dd.axmask, axmask);
-    if (!rc) rc = upload(h, &dd.m0, m0);
-    if (!rc && !fsmask.empty()) rc = upload(h, &dd.fsmask, fsmask);
-    if (!rc) rc = upload(h, &dd.gidx, gidx);
-    if (!rc) rc = upload(h, &dd.start, start);
-    if (!rc) rc = upload(h, &dd.ent, ent);
-    h->in_mesh = false;
-    if (rc) return rc;
-    dd.n_m0 = (int64_t)m0.size();
+// fn(a, b) on ranges of [0, n) over the host's threads
+template <class Fn>
+void parallel_ranges(int64_t n, Fn fn) {
+  const int64_t nt = std::max<int64_t>(1, std::min<int64_t>({(int64_t)std::thread::hardware_concurrency(), 16, n / 4096}));
+  std::vector<std::thread> th;
+  int64_t k = 1;
+  try {
+    for (; k < nt; ++k) th.emplace_back(fn, n * k / nt, n * (k + 1) / nt);
+  } catch (const std::system_error &) {  // no more threads: the rest in this one
+    fn(n * k / nt, n);
   }
-  if ((rc = upload(h, &dd.elinfo, elinfo))) return rc;
-  if ((rc = dalloc(h, &dd.fel, (size_t)nch * 25 * kFlChunk))) return rc;
-  if (d->fluid_src && d->nelsrc > 0) {
-    std::vector<float> s((size_t)8 * 25, 0.f);
-    for (int k = 0; k < d->nelsrc; ++k)
-      for (int q = 0; q < 25; ++q) s[25 * k + q] = d->source_term_fl[q + 25 * k];
-    if ((rc = upload(h, &dd.srcfl, s))) return rc;
-  }
-  return AXG_OK;
+  fn(0, n / nt);
+  for (std::thread &t : th) t.join();
 }
 
-// mesh_part: the element blocks, patch metadata and axial vectors (mesh
-// pool); always: the point words (source and axis flags) and element info
-// words of this solve.  The fluid's arrays: build_fluid_passes.
-int build_domain(axg_handle *h, const axg_mesh_desc *d, bool fluid, bool mesh_part) {
-  const DomainPlan &pl = fluid ? h->pf : h->ps;
-  DomainDev &dd = fluid ? h->df : h->ds;
-  const int64_t nel = pl.nel;
-  if (nel == 0) return AXG_OK;
-  const int pole = d->src_type;
-  const int nonmono = pole != AXG_MONOPOLE;
-  // axial flags and slots
-  std::vector<uint8_t> axial(nel, 0);
-  const int nax = fluid ? d->naxel_fluid : d->naxel_solid;
-  const int32_t *axl = fluid ? d->ax_el_fluid : d->ax_el_solid;
-  for (int k = 0; k < nax; ++k) axial[axl[k] - 1] = 1;
-  std::vector<int> slots;
-  int nt;
-  if (fluid) {
-    nt = nonmono ? 4 : 3;
+// The order of a domain: elements patch by patch in creation order
+// (neighbouring groups then share points, which stay in L1 and L2).
+// Scattered: those of a patch in the reference's order, `last` elements (the
+// fluid's axial ones) at the end, groups of six across patches; points by the
+// first and second patch that hold them.  Patched: those of a patch round by
+// round (the elements of a round share no point), groups within a round.
+void stream_order(const DomainPlan &pl, const int32_t *igloc, const std::vector<uint8_t> &coupled,
+                  const std::vector<uint8_t> *last, bool patched, StreamOrder &o) {
+  const int64_t nel = pl.nel, nglob = pl.nglob;
+  const int32_t np = pl.n_patches;
+  o = StreamOrder();
+  o.patched = patched;
+  o.elem_order.resize(nel);
+  o.group_of_slot.resize(nel);
+  auto add_groups = [&](int64_t a, int64_t b, int wait) {  // slots [a, b)
+    for (int64_t s = a; s < b; s += kGrp) {
+      const int n = (int)std::min<int64_t>(kGrp, b - s);
+      for (int q = 0; q < n; ++q) o.group_of_slot[s + q] = (int32_t)o.groups.size();
+      o.groups.push_back(GroupMeta{(int32_t)s, (uint16_t)n, (uint16_t)wait});
+    }
+  };
+  if (patched) {
+    std::vector<int32_t> launch_of(np);  // the plan's launch position of each patch
+    for (int32_t lp = 0; lp < np; ++lp) launch_of[pl.patch_of_elem[pl.elem_order[pl.meta[lp].elem_start]]] = lp;
+    o.patches.resize(np);
+    int64_t slot = 0;
+    for (int32_t p = 0; p < np; ++p) {
+      const PatchMeta &m = pl.meta[launch_of[p]];
+      PatchInfo &pi = o.patches[p];
+      std::memset(&pi, 0, sizeof pi);
+      pi.group0 = (int32_t)o.groups.size();
+      int r0 = 0;
+      for (int r = 0; r < m.n_rounds; ++r) {
+        const int64_t a = slot;
+        for (int q = r0; q < m.round_end[r]; ++q) o.elem_order[slot++] = pl.elem_order[m.elem_start + q];
+        r0 = m.round_end[r];
+        add_groups(a, slot, (int)o.groups.size() - pi.group0);
+      }
+      pi.n_groups = (uint16_t)(o.groups.size() - pi.group0);
+    }
   } else {
-    slots = solid_slots(pole);
-    nt = (int)slots.size();
+    std::vector<int64_t> fill(np + 1, 0);
+    for (int64_t e = 0; e < nel; ++e) fill[pl.patch_of_elem[e] + 1]++;
+    for (int32_t p = 0; p < np; ++p) fill[p + 1] += fill[p];
+    for (int64_t e = 0; e < nel; ++e) o.elem_order[fill[pl.patch_of_elem[e]]++] = (int32_t)e;
+    if (last)
+      std::stable_partition(o.elem_order.begin(), o.elem_order.end(), [&](int32_t e) { return !(*last)[e]; });
+    add_groups(0, nel, 0);
   }
-  // solid blocks carry the element's point indices and info word inline; the
-  // fluid's element arrays are chunked (fl_at), its slots the plan's launch
-  // order with the axial elements moved to the end, so that the element
-  // pass's warps of 32 slots seldom mix axial and other elements
-  const int bs = fluid ? 25 * nt : solid_block_stride(nt);
-  const int64_t nslots = fluid ? fl_chunks(nel) * kFlChunk : nel;
-  std::vector<float> metric(mesh_part ? (size_t)nslots * bs : 0, 0.f);
-  std::vector<int32_t> elinfo(nel, 0);
-  const std::vector<int> aslots = fluid ? std::vector<int>{0} : axial_slots(pole);
-  const int na = (int)aslots.size();
-  std::vector<float> m0;
-  std::vector<float> fsmask;
-  const bool use_fs = fluid && d->fluid_free_surface_mask != nullptr;
-  if (use_fs && mesh_part) fsmask.resize((size_t)nslots * 25);
-  // source slot of each element
-  std::vector<int8_t> srcslot(nel, -1);
-  if (d->nelsrc > 0 && (bool)d->fluid_src == fluid)
-    for (int k = 0; k < d->nelsrc; ++k) srcslot[d->ielsrc[k] - 1] = (int8_t)k;
-  std::vector<int32_t> order = pl.elem_order;
-  if (fluid) std::stable_partition(order.begin(), order.end(), [&](int32_t e) { return !axial[e]; });
-  int32_t axcount = 0;
-  for (int64_t s = 0; s < nel; ++s) {
-    const int64_t e = order[s];
-    int32_t info = 0;
-    if (axial[e]) {
-      info = axcount + 1;
-      if (mesh_part)
-        for (int q = 0; q < na; ++q)
-          for (int jj = 0; jj < 5; ++jj)
-            m0.push_back(fluid ? (nonmono ? d->m0_w_fl[5 * e + jj] : 0.f) : d->m0_solid[aslots[q]][5 * e + jj]);
-      ++axcount;
-    }
-    if (srcslot[e] >= 0) info |= (srcslot[e] + 1) << 24;
-    elinfo[s] = info;
-    if (!mesh_part) continue;
-    if (fluid) {
-      for (int t = 0; t < nt; ++t)
-        for (int q = 0; q < 25; ++q) metric[fl_at(s, 25 * t + q, bs)] = d->m_fluid[t][25 * e + q];
-      if (use_fs)
-        for (int q = 0; q < 25; ++q) fsmask[fl_at(s, q, 25)] = d->fluid_free_surface_mask[25 * e + q];
-      continue;
-    }
-    float *blk = metric.data() + (size_t)s * bs;
-    for (int t = 0; t < nt; ++t) std::memcpy(blk + 25 * t, d->m_solid[slots[t]] + 25 * e, 25 * sizeof(float));
-    {
-      // the solid kernel reads only the axial slot of this info word
-      std::memcpy(blk + solid_idx_off(nt), &pl.elem_pts[25 * s], 25 * sizeof(uint16_t));
-      std::memcpy(blk + solid_info_off(nt), &info, sizeof(int32_t));
-    }
-  }
-  if (fluid) return build_fluid_passes(h, d, order, dd, mesh_part, metric, elinfo, m0, fsmask, nax, axl);
-  std::vector<uint32_t> pts = pl.pt_words;
-  {
-    // points on the axis: the last writer stores their masked components as
-    // zero, as the reference's axis masks leave its state
-    std::vector<uint8_t> onaxis(fluid ? h->nglob_f : h->nglob_s, 0);
-    const std::vector<int32_t> &ig = fluid ? h->igloc_f : h->igloc_s;
-    for (int k = 0; k < nax; ++k)
-      for (int jj = 0; jj < 5; ++jj) onaxis[ig[25 * (int64_t)(axl[k] - 1) + 5 * jj] - 1] = 1;
-    for (auto &w : pts)
-      if (w != kPtPad && onaxis[w & kPtIndexMask]) w |= kPtAxis;
-    if (mesh_part && nax > 0) {
-      // the components the pole's axis mask zeroes (axis_masked)
-      const uint8_t bits = pole == AXG_MONOPOLE ? 1 : pole == AXG_DIPOLE ? 6 : 7;
-      for (auto &x : onaxis) x = x ? bits : 0;
-      h->in_mesh = true;
-      const int rc = upload(h, &dd.axmask, onaxis);
-      h->in_mesh = false;
-      if (rc) return rc;
-    }
-  }
-  if (!fluid && h->n_src > 0) {
-    // mark the points that carry a solid source term
-    std::vector<uint8_t> issrc(h->nglob_s, 0);
-    // the host copy of the source table is rebuilt here from the descriptor
-    for (int k = 0; k < d->nelsrc; ++k) {
-      const int64_t e = d->ielsrc[k] - 1;
-      for (int q = 0; q < 25; ++q) {
-        bool nz = false;
-        for (int c = 0; c < 3; ++c) nz |= d->source_term_el[q + 25 * k + 200 * c] != 0.f;
-        if (nz) issrc[h->igloc_s[25 * e + q] - 1] = 1;
+  // the first and second patch of each point; a deferred point sorts after
+  // every own point
+  std::vector<int32_t> r0(nglob, np), r1(nglob, np);
+  for (int64_t e = 0; e < nel; ++e) {
+    const int32_t p = pl.patch_of_elem[e];
+    for (int k = 0; k < 25; ++k) {
+      const int64_t g = igloc[25 * e + k] - 1;
+      if (p == r0[g] || p == r1[g]) continue;
+      if (p < r0[g]) {
+        r1[g] = r0[g];
+        r0[g] = p;
+      } else if (p < r1[g]) {
+        r1[g] = p;
       }
     }
-    for (auto &w : pts)
-      if (w != kPtPad && issrc[w & kPtIndexMask]) w |= kPtSource;
   }
-  int rc;
-  if (mesh_part) {
-    h->in_mesh = true;
-    if ((rc = upload(h, &dd.meta, pl.meta)) ||
-        (rc = upload(h, &dd.metric, metric)) || (rc = upload(h, &dd.m0, m0)) ||
-        (use_fs && (rc = upload(h, &dd.fsmask, fsmask)))) {
-      h->in_mesh = false;
-      return rc;
+  std::vector<int32_t> key(nglob, 0);
+  if (patched) {
+    for (int64_t g = 0; g < nglob; ++g) {
+      key[g] = r1[g] < np || r0[g] == np || (!coupled.empty() && coupled[g]);
+      o.n_own += !key[g];
     }
-    h->in_mesh = false;
-    dd.n_m0 = (int64_t)m0.size();
   }
-  if ((rc = upload(h, &dd.pts, pts))) return rc;
-  if ((rc = upload(h, &dd.elinfo, elinfo))) return rc;
+  // three stable counting sorts: second patch, first patch, deferred
+  std::vector<int64_t> fill;
+  auto csort = [&](const std::vector<int32_t> &k, int32_t nkey, const std::vector<int32_t> &in) {
+    fill.assign(nkey + 1, 0);
+    for (int64_t g = 0; g < nglob; ++g) fill[k[g] + 1]++;
+    for (int32_t p = 0; p < nkey; ++p) fill[p + 1] += fill[p];
+    std::vector<int32_t> out(nglob);
+    for (int64_t q = 0; q < nglob; ++q) {
+      const int32_t g = in.empty() ? (int32_t)q : in[q];
+      out[fill[k[g]]++] = g;
+    }
+    return out;
+  };
+  o.old_of_new = csort(key, 2, csort(r0, np + 1, csort(r1, np + 1, {})));
+  o.new_of_old.resize(nglob);
+  for (int64_t n = 0; n < nglob; ++n) o.new_of_old[o.old_of_new[n]] = (int32_t)n;
+  if (!patched) return;
+  // own ranges and deferred lists
+  std::vector<int32_t> seen(nglob, -1);
+  int64_t own = 0;
+  for (int32_t p = 0; p < np; ++p) {
+    PatchInfo &pi = o.patches[p];
+    const GroupMeta &g0 = o.groups[pi.group0], &g1 = o.groups[pi.group0 + pi.n_groups - 1];
+    std::vector<int32_t> def;
+    int n_int = 0;
+    for (int64_t s = g0.slot0; s < g1.slot0 + g1.n; ++s)
+      for (int k = 0; k < 25; ++k) {
+        const int64_t g = igloc[25 * (int64_t)o.elem_order[s] + k] - 1;
+        if (seen[g] == p) continue;
+        seen[g] = p;
+        if (key[g]) def.push_back(o.new_of_old[g]);
+        else ++n_int;
+      }
+    std::sort(def.begin(), def.end());
+    pi.int_start = (int32_t)own;
+    pi.n_int = (uint16_t)n_int;
+    pi.def_start = (int32_t)o.def.size();
+    pi.n_def = (uint16_t)def.size();
+    own += n_int;
+    o.def.insert(o.def.end(), def.begin(), def.end());
+  }
+}
+
+// Solids of more elements than this are patched, unless they carry cg4
+// attenuation.  Below it the scattered contributions (240 or 320 bytes per
+// element) stay in L2 between the two passes and the scattered form's shorter
+// chains win; above it they cost HBM traffic.  Step times, scattered / patched,
+// us, quadrupole: 37.6 / 51.9 at 32 761 elements, 138.7 / 140.0 at 131 044,
+// 261.2 / 256.6 at 262 144, 751 / 717 at 786 432; monopole 45.8 / 46.6 at
+// 65 536, 172 / 155 at 262 144.  The attenuated element pass, with three CTAs
+// per SM, gains nothing from patches: 333 / 387 at 262 144.
+constexpr int64_t kPatchedElems = 131072;
+
+// marks the points that carry a solid source term in the solve's start words
+// of the point pass
+__global__ void flag_source_kernel(int32_t *start, const int32_t *gidx, int32_t n, int32_t p0) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < n && gidx[q] >= p0) start[gidx[q] - p0] |= (int32_t)kStSource;
+}
+
+// mesh_part (mesh pool): the group blocks, axial vectors, free-surface mask
+// and the CSR of the points' copies with its flags (the point has a coupling
+// row, whose number then is its first entry; on the axis).  Always (this
+// solve): the contribution buffer, the solid's start words with the source
+// flags, the fluid's element info words and source terms.
+int build_domain(axg_handle *h, const axg_mesh_desc *d, bool fluid, bool mesh_part,
+                 const std::vector<int32_t> &coupled) {
+  const StreamOrder &o = fluid ? h->of : h->os;
+  DomainDev &dd = fluid ? h->df : h->ds;
+  const int64_t nel = fluid ? h->nel_f : h->nel_s, nglob = fluid ? h->nglob_f : h->nglob_s;
+  if (nel == 0) return AXG_OK;
+  const std::vector<int32_t> &ig = fluid ? h->igloc_f : h->igloc_s;
+  const std::vector<uint8_t> &axial = fluid ? h->axial_f : h->axial_s;
+  const int pole = d->src_type;
+  const bool nonmono = pole != AXG_MONOPOLE;
+  const std::vector<int> slots = fluid ? std::vector<int>{0, 1, 2, 3} : solid_slots(pole);
+  const int nt = fluid ? (nonmono ? 4 : 3) : (int)slots.size();
+  const std::vector<int> aslots = fluid ? std::vector<int>{0} : axial_slots(pole);
+  const int fs = fluid ? kFluidFs : solid_fs(pole);
+  const int64_t p0 = o.n_own, n_pt = nglob - p0;  // the point pass's points
+  dd.n_fel = o.patched ? 4 * (int64_t)o.def.size() : 5 * fs * nel;
+  if (dd.n_fel >= (int64_t)INT32_MAX) return fail(h, AXG_ERR_BAD_DESC, "mesh too large");
+  int rc;
+  std::vector<int32_t> elinfo(nel, 0);
+  {
+    int32_t nax = 0;
+    for (int64_t s = 0; s < nel; ++s)
+      if (axial[o.elem_order[s]]) elinfo[s] = ++nax;
+    if (fluid && d->nelsrc > 0 && d->fluid_src) {
+      std::vector<int8_t> srcslot(nel, -1);
+      for (int k = 0; k < d->nelsrc; ++k) srcslot[d->ielsrc[k] - 1] = (int8_t)k;
+      for (int64_t s = 0; s < nel; ++s)
+        if (srcslot[o.elem_order[s]] >= 0) elinfo[s] |= (srcslot[o.elem_order[s]] + 1) << 24;
+    }
+  }
+  if (mesh_part) {
+    const bool use_fs = fluid && d->fluid_free_surface_mask != nullptr;
+    // a lane's values: index words, then the metric terms (SolidGrp; the
+    // fluid's in rows of four)
+    const int off = o.patched ? 2 : 5, nv = off + 5 * nt, row = fluid ? 4 : 8;
+    const int tail = o.patched && (nv % 8 == 2 || nv % 8 == 4) ? nv % 8 : 0;
+    const int rows = (nv - tail + row - 1) / row;
+    std::vector<float> blocks((size_t)nel * 5 * rows * row, 0.f), tails((size_t)nel * 5 * tail), m0, fsmask;
+    if (use_fs) fsmask.resize((size_t)nel * 25);
+    std::vector<int32_t> patch_of_group(o.patched ? o.groups.size() : 0);
+    for (size_t p = 0; p < o.patches.size(); ++p)
+      for (int q = 0; q < o.patches[p].n_groups; ++q) patch_of_group[o.patches[p].group0 + q] = (int32_t)p;
+    parallel_ranges(nel, [&](int64_t a, int64_t b) {
+      for (int64_t s = a; s < b; ++s) {
+        const int64_t e = o.elem_order[s];
+        const GroupMeta &g = o.group(s);
+        const int ge = (int)(s - g.slot0);
+        for (int j = 0; j < 5; ++j) {
+          auto put = [&](int v, float x) {
+            if (v < rows * row) blocks[grp_at(g, ge, j, v, rows, row)] = x;
+            else tails[((int64_t)g.slot0 * 5 + 5 * ge + j) * tail + v - rows * row] = x;
+          };
+          auto put_word = [&](int v, uint32_t x) {
+            float f;
+            std::memcpy(&f, &x, 4);
+            put(v, f);
+          };
+          uint32_t id[5];
+          for (int i = 0; i < 5; ++i) id[i] = (uint32_t)(ig[25 * e + 5 * j + i] - 1);
+          const uint32_t ax = axial[e] ? kGrpAxial : 0u;
+          if (o.patched) {
+            const PatchInfo &pi = o.patches[patch_of_group[o.group_of_slot[s]]];
+            const int32_t *def = o.def.data() + pi.def_start;
+            for (uint32_t &x : id) {
+              if ((int64_t)x < o.n_own) x -= (uint32_t)pi.int_start;
+              else x = pi.n_int + (uint32_t)(std::lower_bound(def, def + pi.n_def, (int32_t)x) - def);
+            }
+            put_word(0, id[0] | id[1] << 11 | (id[4] & 0x3Fu) << 22 | ax);
+            put_word(1, id[2] | id[3] << 11 | (id[4] >> 6) << 22);
+          } else {
+            id[0] |= ax;
+            for (int i = 0; i < 5; ++i) put_word(i, id[i]);
+          }
+          for (int i = 0; i < 5; ++i)
+            for (int t = 0; t < nt; ++t)
+              put(off + i * nt + t, (fluid ? d->m_fluid[t] : d->m_solid[slots[t]])[25 * e + 5 * j + i]);
+        }
+        if (use_fs) std::memcpy(&fsmask[25 * s], d->fluid_free_surface_mask + 25 * e, 25 * sizeof(float));
+      }
+    });
+    for (int64_t s = 0; s < nel; ++s) {
+      const int64_t e = o.elem_order[s];
+      if (!axial[e]) continue;
+      for (int q : aslots)
+        for (int jj = 0; jj < 5; ++jj)
+          m0.push_back(fluid ? (nonmono ? d->m0_w_fl[5 * e + jj] : 0.f) : d->m0_solid[q][5 * e + jj]);
+    }
+    // per point of the point pass: its coupling row (the fluid keeps its
+    // coupling sums in the force array: no entry), then its copies in slot
+    // order, or its patches' partial sums in patch order
+    std::vector<int64_t> fill(n_pt + 1, 0);
+    if (o.patched) {
+      for (int32_t g : o.def) fill[g - p0 + 1]++;
+    } else {
+      for (int64_t q = 0; q < 25 * nel; ++q) fill[ig[q]]++;
+    }
+    if (!fluid)
+      for (int32_t g : coupled) fill[g - p0 + 1]++;
+    for (int64_t g = 0; g < n_pt; ++g) fill[g + 1] += fill[g];
+    if (fill[n_pt] >= (int64_t)kStMask) return fail(h, AXG_ERR_BAD_DESC, "mesh too large");
+    std::vector<int32_t> start(n_pt + 1), ent((size_t)fill[n_pt]);
+    for (int64_t g = 0; g <= n_pt; ++g) start[g] = (int32_t)fill[g];
+    if (!fluid)
+      for (size_t q = 0; q < coupled.size(); ++q) ent[fill[coupled[q] - p0]++] = (int32_t)q;
+    if (o.patched) {
+      for (size_t q = 0; q < o.def.size(); ++q) ent[fill[o.def[q] - p0]++] = (int32_t)(4 * q);
+    } else {
+      for (int64_t s = 0; s < nel; ++s)
+        for (int k = 0; k < 25; ++k)
+          ent[fill[ig[25 * (int64_t)o.elem_order[s] + k] - 1]++] = (int32_t)((5 * s + k / 5) * fs + k % 5);
+    }
+    std::vector<uint8_t> onaxis(nglob, 0);
+    for (int64_t e = 0; e < nel; ++e)
+      if (axial[e])
+        for (int jj = 0; jj < 5; ++jj) onaxis[ig[25 * e + 5 * jj] - 1] = 1;
+    for (int64_t g = 0; g < n_pt; ++g)
+      if (onaxis[p0 + g]) start[g] |= (int32_t)kStAxis;
+    for (int32_t g : coupled) start[g - p0] |= (int32_t)kStCoupled;
+    std::vector<PatchInfo> patches = o.patches;
+    for (PatchInfo &pi : patches)
+      for (int t = 0; t < pi.n_int; ++t) pi.axis = pi.axis || onaxis[pi.int_start + t];
+    const uint8_t bits = fluid ? (nonmono ? 1 : 0) : pole == AXG_MONOPOLE ? 1 : pole == AXG_DIPOLE ? 6 : 7;
+    std::vector<uint8_t> axmask;
+    if (bits && (fluid ? d->naxel_fluid : d->naxel_solid) > 0) {
+      axmask.resize(nglob);
+      for (int64_t g = 0; g < nglob; ++g) axmask[g] = onaxis[g] ? bits : 0;
+    }
+    dd.n_m0 = (int64_t)m0.size();
+    dd.n_ent = (int64_t)ent.size();
+    h->in_mesh = true;
+    rc = upload(h, &dd.blocks, blocks);
+    if (!rc) rc = upload(h, &dd.tails, tails);
+    if (!rc) rc = upload(h, &dd.patches, patches);
+    if (!rc && o.patched) rc = upload(h, &dd.groups, o.groups);
+    if (!rc) rc = upload(h, &dd.def, o.def);
+    if (!rc) rc = upload(h, &dd.m0, m0);
+    if (!rc && use_fs) rc = upload(h, &dd.fsmask, fsmask);
+    if (!rc && !axmask.empty()) rc = upload(h, &dd.axmask, axmask);
+    if (!rc) rc = upload(h, &dd.start0, start);
+    if (!rc) rc = upload(h, &dd.ent, ent);
+    if (!rc && !fluid) rc = upload(h, &dd.elinfo, elinfo);
+    h->in_mesh = false;
+    if (rc) return rc;
+  }
+  if ((rc = dalloc(h, &dd.fel, (size_t)dd.n_fel))) return rc;
+  if (fluid) {
+    dd.start = dd.start0;
+    dd.srcfl = nullptr;
+    if ((rc = upload(h, &dd.elinfo, elinfo))) return rc;
+    if (d->fluid_src && d->nelsrc > 0) {
+      std::vector<float> v((size_t)8 * 25, 0.f);
+      for (int k = 0; k < d->nelsrc; ++k)
+        for (int q = 0; q < 25; ++q) v[25 * k + q] = d->source_term_fl[q + 25 * k];
+      if ((rc = upload(h, &dd.srcfl, v))) return rc;
+    }
+    return AXG_OK;
+  }
+  if ((rc = dalloc(h, &dd.start, (size_t)n_pt + 1))) return rc;
+  CK(cudaMemcpyAsync(dd.start, dd.start0, (n_pt + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->stream));
+  if (h->n_src > 0)
+    flag_source_kernel<<<(h->n_src + 255) / 256, 256, 0, h->stream>>>(dd.start, h->src_gidx_d, h->n_src, (int32_t)p0);
+  CK(cudaGetLastError());
   return AXG_OK;
 }
 
@@ -634,11 +783,11 @@ CouplingHost make_coupling(std::vector<std::tuple<int32_t, int32_t, float, float
   return c;
 }
 
-// the plain Newmark step: its gather reads the predicted displacement the
-// previous step's last writers stored
-bool lookahead(const axg_handle *h) { return h->scheme == AXG_SCHEME_NEWMARK2 && !h->kahan; }
+// the Newmark step: its gather reads the predicted displacement the previous
+// step's point pass stored
+bool lookahead(const axg_handle *h) { return h->scheme == AXG_SCHEME_NEWMARK2; }
 
-// after a plain Newmark step is queued: its prediction buffers hold the new
+// after a Newmark step is queued: its prediction buffers hold the new
 // displacement and chi, the old displacement buffers the next prediction
 void trade_buffers(axg_handle *h) {
   if (!lookahead(h)) return;
@@ -685,6 +834,7 @@ StateArgs solid_state(axg_handle *h) {
     s.cu[c] = h->kahan ? h->cu_s[c] : nullptr;
     s.cv[c] = h->kahan ? h->cv_s[c] : nullptr;
     s.up[c] = lookahead(h) ? h->sup[c] : nullptr;
+    s.cup[c] = h->kahan ? h->cup_s[c] : nullptr;
   }
   s.inv_mass = h->inv_mass_s;
   s.inv_mass_dp = h->kahan ? h->inv_mass_s_dp : nullptr;
@@ -708,9 +858,10 @@ StateArgs solid_state(axg_handle *h) {
 
 StateArgs fluid_state(axg_handle *h) {
   StateArgs s = solid_state(h);
-  for (int c = 0; c < 3; ++c) s.u[c] = s.v[c] = s.a[c] = s.f[c] = s.cu[c] = s.cv[c] = s.up[c] = nullptr;
+  for (int c = 0; c < 3; ++c) s.u[c] = s.v[c] = s.a[c] = s.f[c] = s.cu[c] = s.cv[c] = s.up[c] = s.cup[c] = nullptr;
   s.cu[0] = h->kahan ? h->cu_f : nullptr;
   s.cv[0] = h->kahan ? h->cv_f : nullptr;
+  s.cup[0] = h->kahan ? h->cup_f : nullptr;
   s.u[0] = h->fu;
   s.up[0] = lookahead(h) ? h->fup : nullptr;
   s.v[0] = h->fv;
@@ -724,9 +875,9 @@ StateArgs fluid_state(axg_handle *h) {
   return s;
 }
 
-// Before a run of the plain Newmark step: the predicted displacement of the
+// Before a run of the Newmark step: the predicted displacement of the
 // current state (it may have been set, reset, restored or advanced by
-// another scheme or mode since the last run).  The last writers keep it from
+// another scheme or mode since the last run).  The point pass keeps it from
 // there on; recomputing it is exact, so runs in pieces match one run.
 void launch_anel_full(axg_handle *h, cudaStream_t s, bool update);
 
@@ -744,72 +895,28 @@ RecWork rec_work(axg_handle *h, const StateArgs &ss) {
   return RecWork{ss, h->rec_gidx_d, h->num_rec, h->seis_it, h->pole, h->nseismo, h->rec, h->iter};
 }
 
-DomainArgs domain_args(const DomainDev &dd, const DomainPlan &pl) {
-  DomainArgs a{};
-  a.n_patches = pl.n_patches;
-  a.n_pts = pl.total_pts;
-  a.n_elem = pl.nel;
-  a.n_m0 = dd.n_m0;
-  a.meta = dd.meta;
-  a.pts = dd.pts;
-  a.elinfo = dd.elinfo;
-  a.metric = dd.metric;
-  a.m0 = dd.m0;
-  a.fsmask = dd.fsmask;
-  a.srcfl = dd.srcfl;
-  return a;
-}
-
-template <int POLE, int MODE, bool ANEL, bool KAHAN = false>
-constexpr int solid_smem_bytes() {
-  constexpr int NC = POLE == POLE_MONO ? 2 : 3;
-  return SolidSmem<NC, solid_block_stride(n_terms(POLE)), solid_stages(ANEL), ANEL ? kAnelSlot : 0,
-                   solid_buffers(MODE, ANEL, KAHAN), solid_row(MODE, ANEL, KAHAN), KAHAN>::bytes;
-}
-
-// sets the kernel's shared-memory attributes; *ctas = resident CTAs on the GPU
-template <class F>
-int prepare_kernel_fn(axg_handle *h, F fn, int bytes, int *ctas) {
-  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  CK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, bytes));
-  if (per_sm < 1) return fail(h, AXG_ERR_CUDA, "solid kernel does not fit on an SM");
-  *ctas = per_sm * h->num_sms;
-  return AXG_OK;
-}
-
-template <int POLE, int MODE, bool ANEL, bool KAHAN>
-int prepare_solid_kernel(axg_handle *h, int *ctas) {
-  return prepare_kernel_fn(h, solid_patch_kernel<POLE, MODE, ANEL, KAHAN>,
-                           solid_smem_bytes<POLE, MODE, ANEL, KAHAN>(), ctas);
-}
-
-// the stiffness kernel and the Newmark kernel the handle's modes select
 template <int POLE>
-int prepare_solid_kernels(axg_handle *h) {
-  int rc = prepare_solid_kernel<POLE, MODE_FORCE, false, false>(h, &h->solid_ctas);
-  if (rc) return rc;
-  int *c = &h->solid_ctas_step;
-  if (h->scheme != AXG_SCHEME_NEWMARK2) {
-    if (h->anel)
-      return h->kahan ? prepare_solid_kernel<POLE, MODE_SYMPLECTIC, true, true>(h, c)
-                      : prepare_solid_kernel<POLE, MODE_SYMPLECTIC, true, false>(h, c);
-    return h->kahan ? prepare_solid_kernel<POLE, MODE_SYMPLECTIC, false, true>(h, c)
-                    : prepare_solid_kernel<POLE, MODE_SYMPLECTIC, false, false>(h, c);
-  }
-  if (h->anel) {
-    return h->kahan ? prepare_solid_kernel<POLE, MODE_NEWMARK, true, true>(h, c)
-                    : prepare_solid_kernel<POLE, MODE_NEWMARK, true, false>(h, c);
-  }
-  return h->kahan ? prepare_solid_kernel<POLE, MODE_NEWMARK, false, true>(h, c)
-                  : prepare_solid_kernel<POLE, MODE_NEWMARK, false, false>(h, c);
+constexpr int force_smem_bytes() {
+  constexpr int NC = POLE == POLE_MONO ? 2 : 3;
+  return SolidSmem<NC, solid_block_stride(n_terms(POLE)), kStages, 2, solid_row()>::bytes;
 }
 
+cudaError_t stream_ctas(int pole, const StreamKernel &k, int *per_sm) {
+  if (pole == AXG_MONOPOLE) return stream_elem_ctas<POLE_MONO>(k, per_sm);
+  if (pole == AXG_DIPOLE) return stream_elem_ctas<POLE_DI>(k, per_sm);
+  return stream_elem_ctas<POLE_QUAD>(k, per_sm);
+}
+
+// the kernel of a launch of the handle's step
+StreamKernel step_kernel(const axg_handle *h, int kind) {
+  return {kind, h->scheme == AXG_SCHEME_NEWMARK2 ? MODE_NEWMARK : MODE_SYMPLECTIC, h->os.patched, h->anel, h->kahan};
+}
+
+// resident CTAs per SM of the element passes the handle's modes select
 int prepare_kernels(axg_handle *h) {
-  if (h->pole == AXG_MONOPOLE) return prepare_solid_kernels<POLE_MONO>(h);
-  if (h->pole == AXG_DIPOLE) return prepare_solid_kernels<POLE_DI>(h);
-  return prepare_solid_kernels<POLE_QUAD>(h);
+  CK(stream_ctas(h->pole, {kElemPass, MODE_FORCE, h->os.patched, false, false}, &h->elem_ctas_force));
+  CK(stream_ctas(h->pole, step_kernel(h, kElemPass), &h->elem_ctas_step));
+  return AXG_OK;
 }
 
 // A launch with programmatic stream serialization: the kernel may start
@@ -832,93 +939,96 @@ void launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t 
   cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-template <int POLE, int MODE, bool ANEL, bool KAHAN>
-void launch_solid_colours(axg_handle *h, cudaStream_t s) {
-  DomainArgs a = domain_args(h->ds, h->ps);
-  StateArgs st = solid_state(h);
-  const int ctas = MODE == MODE_FORCE ? h->solid_ctas : h->solid_ctas_step;
-  for (int c = 0; c < h->ps.n_colours; ++c) {
-    a.patch_begin = h->ps.colour_start[c];
-    const int n = h->ps.colour_start[c + 1] - h->ps.colour_start[c];
-    const int grid = std::min(n, ctas);
-    a.fx = MODE == MODE_NEWMARK && h->anel_full ? h->fx : nullptr;
-    launch_pdl(solid_patch_kernel<POLE, MODE, ANEL, KAHAN>, grid, kThreads, solid_smem_bytes<POLE, MODE, ANEL, KAHAN>(),
-               s, a, st, h->spec, n, h->an);
-  }
-}
-
-template <int POLE, int MODE>
-void launch_solid_pole(axg_handle *h, cudaStream_t s) {
-  if (MODE == MODE_FORCE) {
-    launch_solid_colours<POLE, MODE_FORCE, false, false>(h, s);
-  } else if (h->anel) {
-    if (h->kahan) launch_solid_colours<POLE, MODE_NEWMARK, true, true>(h, s);
-    else launch_solid_colours<POLE, MODE_NEWMARK, true, false>(h, s);
-  } else {
-    if (h->kahan) launch_solid_colours<POLE, MODE_NEWMARK, false, true>(h, s);
-    else launch_solid_colours<POLE, MODE_NEWMARK, false, false>(h, s);
-  }
-}
-
-template <int MODE>
-void launch_solid(axg_handle *h, cudaStream_t s) {
-  if (h->pole == AXG_MONOPOLE) launch_solid_pole<POLE_MONO, MODE>(h, s);
-  else if (h->pole == AXG_DIPOLE) launch_solid_pole<POLE_DI, MODE>(h, s);
-  else launch_solid_pole<POLE_QUAD, MODE>(h, s);
-}
-
-__global__ void zero_points_kernel(const int32_t *gidx, int32_t n, float *f0, float *f1, float *f2) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int g = gidx[q];
-  f0[g] = 0.f;
-  if (f1) f1[g] = 0.f;
-  f2[g] = 0.f;
-}
-
-FluidArgs fluid_args(axg_handle *h) {
-  const DomainDev &dd = h->df;
-  FluidArgs a{};
-  a.gidx = dd.gidx;
-  a.metric = dd.metric;
+StreamDomain stream_domain(const DomainDev &dd, int64_t nel, int64_t nglob) {
+  StreamDomain a{};
+  a.blocks = dd.blocks;
+  a.tails = dd.tails;
   a.elinfo = dd.elinfo;
   a.m0 = dd.m0;
-  a.fsmask = dd.fsmask;
   a.srcfl = dd.srcfl;
+  a.fel = dd.fel;
   a.start = dd.start;
   a.ent = dd.ent;
-  a.fel = dd.fel;
-  a.nel = h->nel_f;
-  a.nglob = h->nglob_f;
+  a.patches = dd.patches;
+  a.groups = dd.groups;
+  a.def = dd.def;
+  a.nel = nel;
+  a.nglob = nglob;
   a.n_m0 = dd.n_m0;
+  a.n_ent = dd.n_ent;
+  a.n_fel = dd.n_fel;
   return a;
 }
 
-// CTAs of the fluid's element pass: one thread per element
-unsigned fluid_elem_grid(int64_t nel) {
-  return (unsigned)std::max<int64_t>(1, (nel + kFlElemThreads - 1) / kFlElemThreads);
+// A mesh whose element blocks do not fit L2 streams them from HBM once per
+// step; a smaller one finds them there.
+constexpr int64_t kL2Resident = 64 << 20;
+
+// the arguments all launches of a step (a stage) share
+StreamWork stream_work(axg_handle *h, int mode, const StateArgs &ss, const StateArgs &fs) {
+  StreamWork w{};
+  w.ds = stream_domain(h->ds, h->nel_s, h->nglob_s);
+  w.ds.aux = mode == MODE_NEWMARK && h->anel_full ? h->fx : nullptr;
+  w.ds.n_patches = (int32_t)h->os.patches.size();
+  w.ds.n_def = (int64_t)h->os.def.size();
+  for (int32_t p : h->src_patches) w.ds.src_patch[w.ds.n_src_patch++] = p;
+  w.solid = ss;
+  w.axmask = h->ds.axmask;
+  w.cg = h->cg;
+  w.iter_p = h->iter_p;
+  w.p0 = (int32_t)h->os.n_own;
+  const int64_t bytes = h->nel_s * 100 * (n_terms(h->pole) + 1);
+  if (bytes > kL2Resident) w.prefetch = (mode == MODE_FORCE ? h->elem_ctas_force : h->elem_ctas_step) * h->num_sms;
+  if (mode == MODE_FORCE) return w;
+  w.rec = rec_work(h, ss);
+  if (h->nel_f > 0) {
+    w.df = stream_domain(h->df, h->nel_f, h->nglob_f);
+    // symplectic_time_loop applies no free-surface mask
+    w.df.aux = mode == MODE_NEWMARK ? h->df.fsmask : nullptr;
+    w.fluid = fs;
+    w.to_fluid = h->to_fluid;
+    w.to_solid = h->to_solid;
+    w.ffl = h->ff;
+  }
+  return w;
 }
 
-// The fluid of a Newmark step or a symplectic stage: the element pass, then
-// the point pass.
-template <int NONMONO, int MODE, bool KAHAN>
-void launch_fluid_t(axg_handle *h, cudaStream_t s, const StateArgs &fs) {
-  FluidArgs fa = fluid_args(h);
-  if (MODE == MODE_SYMPLECTIC) fa.fsmask = nullptr;  // symplectic_time_loop applies no free-surface mask
-  launch_pdl(fluid_elem_kernel<NONMONO, MODE, KAHAN, One<FluidWork>>, fluid_elem_grid(h->nel_f), kFlElemThreads, 0, s,
-             One<FluidWork>{{fa, fs}, (int32_t)h->nel_f}, h->spec);
-  launch_pdl(fluid_point_kernel<NONMONO, MODE, KAHAN, One<FluidWork>>, (unsigned)((h->nglob_f + 255) / 256), 256, 0,
-             s, One<FluidWork>{{fa, fs}, (int32_t)h->nglob_f});
-}
-template <int MODE>
-void launch_fluid(axg_handle *h, cudaStream_t s, const StateArgs &fs) {
-  if (h->pole == AXG_MONOPOLE) {
-    if (h->kahan) launch_fluid_t<0, MODE, true>(h, s, fs);
-    else launch_fluid_t<0, MODE, false>(h, s, fs);
-  } else {
-    if (h->kahan) launch_fluid_t<1, MODE, true>(h, s, fs);
-    else launch_fluid_t<1, MODE, false>(h, s, fs);
+int32_t ceil_div(int64_t a, int64_t b) { return (int32_t)((a + b - 1) / b); }
+
+// The launches of a step (a stage): fn(kind, work) in order.  The element
+// pass takes the solid, the fluid and the coupling into the fluid; the point
+// pass the solid's and the fluid's points.  The coupling into the solid takes
+// the new fluid acceleration from the fluid's contributions; with absorbing
+// fluid terms, which need the fluid's velocity, the fluid's point pass runs
+// before the solid's in a launch of its own.  The last launch of a Newmark
+// step also records the seismograms and counts the step.
+template <class Fn>
+void stream_launches(const axg_handle *h, int mode, const StreamWork &base, Fn fn) {
+  const bool fluid = mode != MODE_FORCE && h->nel_f > 0;
+  const int32_t nb_fp = fluid ? ceil_div(h->nglob_f, kGrpThreads) : 0;
+  StreamWork w = base;
+  w.nb_se = h->os.patched ? (int32_t)h->os.patches.size() : ceil_div(grp_count(h->nel_s), kGrpWarps);
+  if (fluid) {
+    w.nb_fe = ceil_div(grp_count(h->nel_f), kGrpWarps);
+    w.nb_cp = ceil_div(h->to_fluid.n, kGrpThreads);
   }
+  fn(kElemPass, w);
+  w = base;
+  w.nb_fp = nb_fp;
+  if (fluid && base.fluid.gamma && h->to_solid.n > 0) {
+    fn(kPointPass, w);
+    w.nb_fp = 0;
+  }
+  w.nb_sp = ceil_div(h->nglob_s - h->os.n_own, kGrpThreads);
+  if (mode == MODE_NEWMARK) w.nb_rec = 1;
+  if (stream_blocks(w) > 0) fn(kPointPass, w);
+}
+
+void launch_stream(axg_handle *h, const StreamKernel &k, const StreamWork &w, cudaStream_t s) {
+  const StreamOne p{w};
+  if (h->pole == AXG_MONOPOLE) stream_launch<POLE_MONO>(k, p, h->spec, s);
+  else if (h->pole == AXG_DIPOLE) stream_launch<POLE_DI>(k, p, h->spec, s);
+  else stream_launch<POLE_QUAD>(k, p, h->spec, s);
 }
 
 // Attenuation at every GLL point: with update, the step's memory variables
@@ -926,7 +1036,7 @@ void launch_fluid(axg_handle *h, cudaStream_t s, const StateArgs &fs) {
 // memory variables (before a run)
 template <int POLE>
 void launch_anel_full_pole(axg_handle *h, cudaStream_t s, bool update) {
-  const FullAnelArgs fa{h->an, h->fx, h->sym_gidx, h->sym_axial, h->nel_s};
+  const FullAnelArgs fa{h->an, h->fx, h->slot_gidx, h->slot_axial, h->nel_s};
   const unsigned g = (unsigned)std::min<int64_t>((h->nel_s + kWarps - 1) / kWarps, 16 * (int64_t)h->num_sms);
   if (update) launch_pdl(anel_full_kernel<POLE, true>, g, kThreads, 0, s, fa, solid_state(h), h->spec);
   else anel_full_kernel<POLE, false><<<g, kThreads, 0, s>>>(fa, solid_state(h), h->spec);
@@ -938,10 +1048,10 @@ void launch_anel_full(axg_handle *h, cudaStream_t s, bool update) {
 }
 
 void enqueue_force(axg_handle *h, cudaStream_t s) {
-  if (h->to_solid.n > 0)
-    zero_points_kernel<<<(h->to_solid.n + 255) / 256, 256, 0, s>>>(h->to_solid.pt_gidx, h->to_solid.n, h->sf[0],
-                                                                   h->sf[1], h->sf[2]);
-  launch_solid<MODE_FORCE>(h, s);
+  const StreamWork w = stream_work(h, MODE_FORCE, solid_state(h), StateArgs{});
+  stream_launches(h, MODE_FORCE, w, [&](int kind, const StreamWork &x) {
+    launch_stream(h, {kind, MODE_FORCE, h->os.patched, false, false}, x, s);
+  });
 }
 
 void enqueue_step_symplectic(axg_handle *h, cudaStream_t s);
@@ -951,54 +1061,11 @@ void enqueue_step(axg_handle *h, cudaStream_t s) {
     enqueue_step_symplectic(h, s);
     return;
   }
-  StateArgs ss = solid_state(h), fs = fluid_state(h);
-  if (h->nel_f > 0) {
-    if (h->to_fluid.n > 0) {
-      const unsigned nb = (h->to_fluid.n + 255) / 256;
-      const One<ToFluidWork> w{{h->to_fluid, ss, h->ff, h->ds.axmask}, h->to_fluid.n};
-      if (h->pole == AXG_DIPOLE) launch_pdl(couple_to_fluid_kernel<1, One<ToFluidWork>>, nb, 256, 0, s, w);
-      else launch_pdl(couple_to_fluid_kernel<0, One<ToFluidWork>>, nb, 256, 0, s, w);
-    }
-    launch_fluid<MODE_NEWMARK>(h, s, fs);
-    if (h->to_solid.n > 0) {
-      const unsigned nb = (h->to_solid.n + 255) / 256;
-      const One<ToSolidWork> w{{h->to_solid, fs, ss}, h->to_solid.n};
-      if (h->pole == AXG_MONOPOLE) launch_pdl(couple_to_solid_kernel<POLE_MONO, One<ToSolidWork>>, nb, 256, 0, s, w);
-      else if (h->pole == AXG_DIPOLE) launch_pdl(couple_to_solid_kernel<POLE_DI, One<ToSolidWork>>, nb, 256, 0, s, w);
-      else launch_pdl(couple_to_solid_kernel<POLE_QUAD, One<ToSolidWork>>, nb, 256, 0, s, w);
-    }
-  }
-  launch_solid<MODE_NEWMARK>(h, s);
+  const StreamWork w = stream_work(h, MODE_NEWMARK, solid_state(h), fluid_state(h));
+  stream_launches(h, MODE_NEWMARK, w,
+                  [&](int kind, const StreamWork &x) { launch_stream(h, step_kernel(h, kind), x, s); });
   trade_buffers(h);  // the state after the step
   if (h->anel_full) launch_anel_full(h, s, true);  // the memory variables from the stored displacement
-  launch_pdl(receivers_kernel<One<RecWork>>, 1, 256, 0, s, One<RecWork>{rec_work(h, solid_state(h)), 1});
-}
-
-// One step of symplectic_time_loop (SOLVER/time_evol_wave.F90:587-727):
-// per stage the drift (on the gathers), fluid stiffness and the coupling
-// into it, solid stiffness, the coupling into the solid, the kicks (by the
-// last writers); then the final drift and the seismograms.
-template <int POLE, bool ANEL, bool KAHAN>
-void launch_solid_symplectic_modes(axg_handle *h, cudaStream_t s, const StateArgs &st) {
-  DomainArgs a = domain_args(h->ds, h->ps);
-  for (int c = 0; c < h->ps.n_colours; ++c) {
-    a.patch_begin = h->ps.colour_start[c];
-    const int n = h->ps.colour_start[c + 1] - h->ps.colour_start[c];
-    solid_patch_kernel<POLE, MODE_SYMPLECTIC, ANEL, KAHAN>
-        <<<std::min(n, h->solid_ctas_step), kThreads, solid_smem_bytes<POLE, MODE_SYMPLECTIC, ANEL, KAHAN>(), s>>>(
-            a, st, h->spec, n, h->an);
-  }
-}
-
-template <int POLE>
-void launch_solid_symplectic(axg_handle *h, cudaStream_t s, const StateArgs &st) {
-  if (h->anel) {
-    if (h->kahan) launch_solid_symplectic_modes<POLE, true, true>(h, s, st);
-    else launch_solid_symplectic_modes<POLE, true, false>(h, s, st);
-  } else {
-    if (h->kahan) launch_solid_symplectic_modes<POLE, false, true>(h, s, st);
-    else launch_solid_symplectic_modes<POLE, false, false>(h, s, st);
-  }
 }
 
 // the solid and fluid state of stage i of a symplectic step
@@ -1027,47 +1094,32 @@ int32_t drift_points(const axg_handle *h) {
   return (int32_t)std::max(h->nglob_s, h->nel_f > 0 ? h->nglob_f : 0);
 }
 
-template <int POLE>
-void launch_anel_memvar(axg_handle *h, cudaStream_t s) {
-  const unsigned g = (unsigned)std::min<int64_t>((h->nel_s + kWarps - 1) / kWarps, 16 * (int64_t)h->num_sms);
-  anel_memvar_kernel<POLE><<<g, kThreads, 0, s>>>(h->an, h->sym_gidx, h->sym_axial, solid_state(h), h->nel_s,
-                                                  h->spec);
-}
 // the memory variables from the drifted displacement, once per symplectic step
-void launch_anel_memvar_pole(axg_handle *h, cudaStream_t s) {
-  if (h->pole == AXG_MONOPOLE) launch_anel_memvar<POLE_MONO>(h, s);
-  else if (h->pole == AXG_DIPOLE) launch_anel_memvar<POLE_DI>(h, s);
-  else launch_anel_memvar<POLE_QUAD>(h, s);
+void launch_anel_memvar(axg_handle *h, cudaStream_t s) {
+  StreamOne p{stream_work(h, MODE_SYMPLECTIC, solid_state(h), fluid_state(h))};
+  p.w.memvar_gidx = h->slot_gidx;
+  const int32_t n = (int32_t)h->os.groups.size();
+  if (h->pole == AXG_MONOPOLE) stream_memvar<POLE_MONO>(h->os.patched, p, h->spec, n, s);
+  else if (h->pole == AXG_DIPOLE) stream_memvar<POLE_DI>(h->os.patched, p, h->spec, n, s);
+  else stream_memvar<POLE_QUAD>(h->os.patched, p, h->spec, n, s);
 }
 
+// One step of symplectic_time_loop (SOLVER/time_evol_wave.F90:587-727):
+// per stage the drift (on the gathers), fluid stiffness and the coupling
+// into it, solid stiffness, the coupling into the solid and the kicks (in the
+// point pass); then the final drift and the seismograms.
 void enqueue_step_symplectic(axg_handle *h, cudaStream_t s) {
   for (int i = 0; i < h->nstages; ++i) {
     StateArgs ss, fs;
     symplectic_stage_states(h, i, ss, fs);
-    if (h->nel_f > 0) {
-      if (h->to_fluid.n > 0) {
-        const int nb = (h->to_fluid.n + 255) / 256;
-        const One<ToFluidWork> w{{h->to_fluid, ss, h->ff, h->ds.axmask}, h->to_fluid.n};
-        if (h->pole == AXG_DIPOLE) couple_to_fluid_kernel<1><<<nb, 256, 0, s>>>(w);
-        else couple_to_fluid_kernel<0><<<nb, 256, 0, s>>>(w);
-      }
-      launch_fluid<MODE_SYMPLECTIC>(h, s, fs);
-      if (h->to_solid.n > 0) {
-        const int nb = (h->to_solid.n + 255) / 256;
-        const One<ToSolidWork> w{{h->to_solid, fs, ss}, h->to_solid.n};
-        if (h->pole == AXG_MONOPOLE) couple_to_solid_kernel<POLE_MONO><<<nb, 256, 0, s>>>(w);
-        else if (h->pole == AXG_DIPOLE) couple_to_solid_kernel<POLE_DI><<<nb, 256, 0, s>>>(w);
-        else couple_to_solid_kernel<POLE_QUAD><<<nb, 256, 0, s>>>(w);
-      }
-    }
-    if (h->pole == AXG_MONOPOLE) launch_solid_symplectic<POLE_MONO>(h, s, ss);
-    else if (h->pole == AXG_DIPOLE) launch_solid_symplectic<POLE_DI>(h, s, ss);
-    else launch_solid_symplectic<POLE_QUAD>(h, s, ss);
+    const StreamWork w = stream_work(h, MODE_SYMPLECTIC, ss, fs);
+    stream_launches(h, MODE_SYMPLECTIC, w,
+                    [&](int kind, const StreamWork &x) { launch_stream(h, step_kernel(h, kind), x, s); });
   }
   const int32_t n = drift_points(h);
-  drift_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(One<DriftWork>{drift_work(h), n});
-  if (h->anel) launch_anel_memvar_pole(h, s);
-  receivers_kernel<<<1, 256, 0, s>>>(One<RecWork>{rec_work(h, solid_state(h)), 1});
+  launch_pdl(drift_kernel<One<DriftWork>>, (unsigned)((n + 255) / 256), 256, 0, s, One<DriftWork>{drift_work(h), n});
+  if (h->anel) launch_anel_memvar(h, s);
+  launch_pdl(receivers_kernel<One<RecWork>>, 1, 256, 0, s, One<RecWork>{rec_work(h, solid_state(h)), 1});
 }
 
 // a CUDA graph of nsteps steps into *exec (replacing what it held).  The
@@ -1312,19 +1364,21 @@ void sls_fast_correct(const double *y, double *yp, int n) {
 //    rounded to float once;
 //  * per element (launch order) the cg4 constants and the two row indices;
 //  * the per-element state, zeroed by axg_reset.
-// the element slots' points and axis flags (launch order), for the kernels
-// that visit elements outside the patch kernel
+// floats of the cg4 state
+int64_t cg_floats(const axg_handle *h) { return 4 * h->nel_s * (int64_t)cg_state_floats(h->nsls); }
+
+// the element slots' points and axis flags, for the pass over all GLL points
 int upload_slot_points(axg_handle *h) {
-  if (h->sym_gidx) return AXG_OK;
+  if (h->slot_gidx) return AXG_OK;
   std::vector<int32_t> g(25 * (size_t)h->nel_s);
   std::vector<uint8_t> ax(h->nel_s);
-  for (int64_t e = 0; e < h->nel_s; ++e) {
-    const int64_t sl = h->slot_of_elem_s[e];
+  for (int64_t sl = 0; sl < h->nel_s; ++sl) {
+    const int64_t e = h->os.elem_order[sl];
     for (int k = 0; k < 25; ++k) g[25 * sl + k] = h->igloc_s[25 * e + k] - 1;
     ax[sl] = h->axial_s[e];
   }
   int rc;
-  if ((rc = upload(h, &h->sym_gidx, g)) || (rc = upload(h, &h->sym_axial, ax))) return rc;
+  if ((rc = upload(h, &h->slot_gidx, g)) || (rc = upload(h, &h->slot_axial, ax))) return rc;
   return AXG_OK;
 }
 
@@ -1336,7 +1390,7 @@ int build_anel_full(axg_handle *h, const axg_mesh_desc *d, bool mesh_part, RowFn
                     const std::map<float, int32_t> &qrow) {
   const int nsls = d->n_sls;
   const int64_t nel = h->nel_s;
-  const DomainPlan &pl = h->ps;
+  const StreamOrder &pl = h->os;
   std::vector<float> consts((size_t)nel * kFullConst, 0.f);
   const float *pt[12] = {d->delta_mu, d->delta_kappa, d->Y, d->V_s_eta, d->V_s_xi, d->V_z_eta, d->V_z_xi,
                          d->DsDeta_over_J_sol, d->DzDeta_over_J_sol, d->DsDxi_over_J_sol, d->DzDxi_over_J_sol,
@@ -1357,8 +1411,6 @@ int build_anel_full(axg_handle *h, const axg_mesh_desc *d, bool mesh_part, RowFn
   h->an.state_stride = full_state_stride(nsls);
   h->an.n_q = (int32_t)qrow.size();
   for (int j = 0; j < kMaxSls; ++j) h->an.ex[j] = j < nsls ? (float)d->exp_w_j_deltat[j] : 0.f;
-  h->slot_of_elem_s.assign(nel, 0);
-  for (int64_t s = 0; s < nel; ++s) h->slot_of_elem_s[pl.elem_order[s]] = (int32_t)s;
   int rc;
   float *cp = nullptr, *qp = nullptr;
   if (mesh_part) {
@@ -1378,7 +1430,7 @@ int build_anel_full(axg_handle *h, const axg_mesh_desc *d, bool mesh_part, RowFn
 int build_anel(axg_handle *h, const axg_mesh_desc *d, bool mesh_part) {
   const int nsls = d->n_sls;
   const int64_t nel = h->nel_s;
-  const DomainPlan &pl = h->ps;
+  const StreamOrder &pl = h->os;
   std::map<float, int32_t> qrow;
   std::vector<float> qtab;
   auto row = [&](float Q) {
@@ -1400,28 +1452,26 @@ int build_anel(axg_handle *h, const axg_mesh_desc *d, bool mesh_part) {
     return r;
   };
   if (h->anel_full) return build_anel_full(h, d, mesh_part, row, qtab, qrow);
-  std::vector<float> consts((size_t)nel * kAnelConst, 0.f);
+  std::vector<float> consts((size_t)nel * 48);
+  std::vector<int2> qrows((size_t)nel);
   const float *fields[11] = {d->delta_mu_cg4, d->delta_kappa_cg4, d->Y_cg4,  d->V_s_eta_cg4,
                              d->V_s_xi_cg4,   d->V_z_eta_cg4,    d->V_z_xi_cg4, d->DsDeta_over_J_sol_cg4,
                              d->DzDeta_over_J_sol_cg4, d->DsDxi_over_J_sol_cg4, d->DzDxi_over_J_sol_cg4};
   const int cg_pt[4] = {1 + 5 * 1, 1 + 5 * 3, 3 + 5 * 1, 3 + 5 * 3};
   for (int64_t s = 0; s < nel; ++s) {
     const int64_t e = pl.elem_order[s];
-    float *c = consts.data() + (size_t)s * kAnelConst;
-    for (int f = 0; f < 11; ++f)
-      for (int k = 0; k < 4; ++k) c[4 * f + k] = fields[f][4 * e + k];
-    for (int k = 0; k < 4; ++k) c[A_INVS + k] = d->inv_s_solid[25 * e + cg_pt[k]];
-    const int32_t qm = row(d->Q_mu[e]), qk = row(d->Q_kappa[e]);
-    std::memcpy(c + A_QMU, &qm, 4);
-    std::memcpy(c + A_QKA, &qk, 4);
+    const GroupMeta &g = pl.group(s);
+    const int ge = (int)(s - g.slot0);
+    for (int k = 0; k < 4; ++k) {
+      for (int f = 0; f < 11; ++f) consts[cg_const_at(g, ge, k, f)] = fields[f][4 * e + k];
+      consts[cg_const_at(g, ge, k, 11)] = d->inv_s_solid[25 * e + cg_pt[k]];
+    }
+    qrows[s] = make_int2(row(d->Q_mu[e]), row(d->Q_kappa[e]));
   }
   h->nsls = nsls;
-  h->an.nsls = nsls;
-  h->an.state_stride = anel_state_stride(nsls);
-  h->an.n_q = (int32_t)qrow.size();
-  for (int j = 0; j < kMaxSls; ++j) h->an.ex[j] = j < nsls ? (float)d->exp_w_j_deltat[j] : 0.f;
-  h->slot_of_elem_s.assign(nel, 0);
-  for (int64_t s = 0; s < nel; ++s) h->slot_of_elem_s[pl.elem_order[s]] = (int32_t)s;
+  h->cg.nsls = nsls;
+  h->cg.n_q = (int32_t)qrow.size();
+  for (int j = 0; j < kMaxSls; ++j) h->cg.ex[j] = j < nsls ? (float)d->exp_w_j_deltat[j] : 0.f;
   int rc;
   float *cp = nullptr, *qp = nullptr;
   if (mesh_part) {  // the per-element constants belong to the mesh
@@ -1429,12 +1479,13 @@ int build_anel(axg_handle *h, const axg_mesh_desc *d, bool mesh_part) {
     rc = upload(h, &cp, consts);
     h->in_mesh = false;
     if (rc) return rc;
-    h->an.consts = cp;
+    h->cg.consts = cp;
   }
-  if ((rc = upload(h, &qp, qtab))) return rc;  // depends on dt: this solve's
-  h->an.qtab = qp;
-  if ((rc = dalloc(h, &h->an.state, (size_t)nel * h->an.state_stride))) return rc;
-  return AXG_OK;
+  int2 *qd = nullptr;
+  if ((rc = upload(h, &qp, qtab)) || (rc = upload(h, &qd, qrows))) return rc;  // the table depends on dt: this solve's
+  h->cg.qtab = qp;
+  h->cg.q = qd;
+  return dalloc(h, &h->cg.state, (size_t)cg_floats(h));
 }
 
 }  // namespace
@@ -1443,6 +1494,22 @@ extern "C" int axg_reset(axg_handle *h);
 extern "C" int axg_device_count(void);
 
 namespace {
+// the launches of a step and of a stiffness + assembly
+void count_launches(axg_handle *h) {
+  auto count = [&](int mode) {
+    StateArgs fs{};
+    fs.gamma = h->gamma_f;
+    StreamWork w{};
+    w.fluid = fs;
+    int64_t n = 0;
+    stream_launches(h, mode, w, [&](int, const StreamWork &) { ++n; });
+    return n;
+  };
+  h->kernels_per_force = count(MODE_FORCE);
+  if (h->scheme == AXG_SCHEME_NEWMARK2) h->kernels_per_step = count(MODE_NEWMARK) + (h->anel_full ? 1 : 0);
+  else h->kernels_per_step = h->nstages * count(MODE_SYMPLECTIC) + 2 + (h->anel ? 1 : 0);
+}
+
 // share: an existing handle on the same mesh (axg_create_sharing) whose
 // plans and mesh-level device buffers are used instead of building new ones
 int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share = nullptr) {
@@ -1479,8 +1546,8 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
         if (ig[p] < 1 || ig[p] > nglob || mine[p] != nofo[ig[p] - 1] + 1) return false;
       return true;
     };
-    if (!same(share->igloc_s, d->igloc_solid, 25 * h->nel_s, h->nglob_s, share->ps.new_of_old) ||
-        (h->nel_f > 0 && !same(share->igloc_f, d->igloc_fluid, 25 * h->nel_f, h->nglob_f, share->pf.new_of_old)))
+    if (!same(share->igloc_s, d->igloc_solid, 25 * h->nel_s, h->nglob_s, share->os.new_of_old) ||
+        (h->nel_f > 0 && !same(share->igloc_f, d->igloc_fluid, 25 * h->nel_f, h->nglob_f, share->of.new_of_old)))
       return fail(h, AXG_ERR_BAD_DESC, "axg_create_sharing: the global numbering differs from the handle's mesh");
     h->igloc_s = share->igloc_s;
     h->igloc_f = share->igloc_f;
@@ -1490,6 +1557,9 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
     h->pre_f = share->pre_f;
     h->ps = share->ps;
     h->pf = share->pf;
+    h->os = share->os;
+    h->of = share->of;
+    h->slot_of_elem_s = share->slot_of_elem_s;
     h->patch_elems = share->patch_elems;
     h->growth = share->growth;
   } else {
@@ -1541,13 +1611,26 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
     perr = validate_plan(h->igloc_s.data(), h->nel_s, h->nglob_s, h->pre_s, h->ps);
     if (!perr.empty()) return fail(h, AXG_ERR_BAD_DESC, "solid plan invalid: " + perr);
 #endif
-    // from here on points carry the plans' internal numbers
-    for (int32_t &g : h->igloc_s) g = h->ps.new_of_old[g - 1] + 1;
-    for (int32_t &g : h->igloc_f) g = h->pf.new_of_old[g - 1] + 1;
-    for (int32_t &g : cs.pt_gidx) g = h->ps.new_of_old[g];
-    for (int32_t &g : cs.src_gidx) g = h->pf.new_of_old[g];
-    for (int32_t &g : cf.pt_gidx) g = h->pf.new_of_old[g];
-    for (int32_t &g : cf.src_gidx) g = h->ps.new_of_old[g];
+    stream_order(h->ps, h->igloc_s.data(), h->pre_s, nullptr, !h->anel && h->nel_s > kPatchedElems, h->os);
+    // the fluid's axial elements at the end, so that its warps seldom mix
+    // axial and other elements
+    if (h->nel_f > 0) stream_order(h->pf, h->igloc_f.data(), h->pre_f, &h->axial_f, false, h->of);
+    for (DomainPlan *p : {&h->ps, &h->pf}) {  // what only the patch kernel of the no-allocation entry point reads
+      for (std::vector<int32_t> *v : {&p->elem_order, &p->new_of_old, &p->old_of_new}) std::vector<int32_t>().swap(*v);
+      std::vector<uint32_t>().swap(p->pt_words);
+      std::vector<uint16_t>().swap(p->elem_pts);
+    }
+    if (h->anel || h->anel_full) {
+      h->slot_of_elem_s.resize(h->nel_s);
+      for (int64_t s = 0; s < h->nel_s; ++s) h->slot_of_elem_s[h->os.elem_order[s]] = (int32_t)s;
+    }
+    // from here on points carry the internal numbers
+    for (int32_t &g : h->igloc_s) g = h->os.new_of_old[g - 1] + 1;
+    for (int32_t &g : h->igloc_f) g = h->of.new_of_old[g - 1] + 1;
+    for (int32_t &g : cs.pt_gidx) g = h->os.new_of_old[g];
+    for (int32_t &g : cs.src_gidx) g = h->of.new_of_old[g];
+    for (int32_t &g : cf.pt_gidx) g = h->of.new_of_old[g];
+    for (int32_t &g : cf.src_gidx) g = h->os.new_of_old[g];
   }
 
   // receivers and the solid source table
@@ -1581,6 +1664,15 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
     }
   }
   h->n_src = (int32_t)src_g.size();
+  for (int32_t g : src_g) {
+    if (g >= h->os.n_own) continue;
+    const auto it = std::upper_bound(h->os.patches.begin(), h->os.patches.end(), g,
+                                     [](int32_t x, const PatchInfo &p) { return x < p.int_start; });
+    // (a patch without own points starts where the next does)
+    int32_t p = (int32_t)(it - h->os.patches.begin()) - 1;
+    while (g >= h->os.patches[p].int_start + h->os.patches[p].n_int) --p;
+    if (std::find(h->src_patches.begin(), h->src_patches.end(), p) == h->src_patches.end()) h->src_patches.push_back(p);
+  }
 
   // ---- device
   CK(cudaGetDevice(&h->device));
@@ -1609,6 +1701,7 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
     h->to_fluid = share->to_fluid;
     h->to_solid = share->to_solid;
     h->an.consts = share->an.consts;
+    h->cg.consts = share->cg.consts;
     h->dev_bytes = h->mesh->bytes;
   } else {
     h->mesh = std::make_shared<MeshPool>();
@@ -1631,8 +1724,9 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
     h->to_solid.nglob_recv = h->nglob_s;
     h->to_solid.nglob_send = h->nglob_f;
   }
-  if ((rc = build_domain(h, d, false, !share))) return rc;
-  if ((rc = build_domain(h, d, true, !share))) return rc;
+  if ((rc = upload(h, &h->src_gidx_d, src_g))) return rc;
+  if ((rc = build_domain(h, d, false, !share, cs.pt_gidx))) return rc;
+  if ((rc = build_domain(h, d, true, !share, cf.pt_gidx))) return rc;
   const bool mono = h->pole == AXG_MONOPOLE;
   for (int c = 0; c < 3; ++c) {
     if (mono && c == 1) continue;
@@ -1652,17 +1746,15 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
   if ((rc = upload(h, &h->stf, stf))) return rc;
   if ((rc = dalloc(h, &h->rec, (size_t)h->nseismo * 3 * std::max(h->num_rec, 1)))) return rc;
   if ((rc = upload(h, &h->rec_gidx_d, h->rec_gidx))) return rc;
-  if ((rc = upload(h, &h->src_gidx_d, src_g))) return rc;
   if ((rc = upload(h, &h->src_val_d, src_v))) return rc;
   if (!src_v_dp.empty() && (rc = upload(h, &h->src_val_dp_d, src_v_dp))) return rc;
   if ((rc = dalloc(h, &h->iter, 4))) return rc;
   h->blowup = h->iter + 1;
   h->errw = h->iter + 2;
+  h->iter_p = h->iter + 3;
   if ((h->anel || h->anel_full) && (rc = build_anel(h, d, !share))) return rc;
   if ((rc = prepare_kernels(h))) return rc;
-  h->kernels_per_force = h->ps.n_colours + (h->to_solid.n > 0 ? 1 : 0);
-  h->kernels_per_step = h->ps.n_colours + 1 + (h->anel_full ? 1 : 0) +
-                        (h->nel_f > 0 ? 2 + (h->to_fluid.n > 0) + (h->to_solid.n > 0) : 0);
+  count_launches(h);
   return axg_reset(h);
 }
 }  // namespace
@@ -1694,8 +1786,8 @@ NoAllocDevice g_noalloc_dev[kNoAllocMaxDevices];
 
 template <int POLE>
 int noalloc_prepare_kernel(int nsm, int *cap) {
-  auto fn = solid_patch_kernel<POLE, MODE_FORCE, false, false>;
-  const int bytes = solid_smem_bytes<POLE, MODE_FORCE, false, false>();
+  auto fn = solid_patch_kernel<POLE>;
+  const int bytes = force_smem_bytes<POLE>();
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   int per_sm = 0;
@@ -1762,9 +1854,7 @@ void noalloc_launch(const DomainArgs &a0, const StateArgs &st, const SpecDev &sp
   for (int c = 0; c < pl.n_colours; ++c) {
     a.patch_begin = pl.colour_start[c];
     const int n = pl.colour_start[c + 1] - pl.colour_start[c];
-    solid_patch_kernel<POLE, MODE_FORCE, false, false>
-        <<<std::min(n, cap), kThreads, solid_smem_bytes<POLE, MODE_FORCE, false, false>(), 0>>>(a, st, sp, n,
-                                                                                           AnelArgs{});
+    solid_patch_kernel<POLE><<<std::min(n, cap), kThreads, force_smem_bytes<POLE>(), 0>>>(a, st, sp, n);
   }
 }
 
@@ -1899,19 +1989,31 @@ int anel_state_io(axg_handle *h, int field, float *out, const float *in) {
   const int64_t nel = h->nel_s, stride = h->an.state_stride;
   const int nsls = h->nsls;
   const int np = h->anel_full ? 25 : 4;  // points per element with memory variables
-  int off = 0, len = 6 * np * nsls;  // floats per element of this field, and where they start in the state
+  int off = 0, len = 6 * np * nsls;  // floats per element of this field, and where they start in the reference's order
   if (field == AXG_FIELD_ATT_SRC_TR) off = 6 * np * nsls, len = np;
   if (field == AXG_FIELD_ATT_SRC_DEV) off = 6 * np * nsls + np, len = 6 * np;
-  std::vector<float> st((size_t)nel * stride);
-  CK(cudaMemcpyAsync(st.data(), h->an.state, st.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+  float *dev = h->anel_full ? h->an.state : h->cg.state;
+  std::vector<float> st((size_t)(h->anel_full ? nel * stride : cg_floats(h)));
+  CK(cudaMemcpyAsync(st.data(), dev, st.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   for (int64_t e = 0; e < nel; ++e) {
-    float *blk = st.data() + (size_t)h->slot_of_elem_s[e] * stride + off;
-    if (out) std::memcpy(out + (size_t)e * len, blk, len * sizeof(float));
-    else std::memcpy(blk, in + (size_t)e * len, len * sizeof(float));
+    const int64_t s = h->slot_of_elem_s[e];
+    for (int x = 0; x < len; ++x) {
+      int64_t at = s * stride + off + x;
+      if (!h->anel_full) {
+        // entry x of (1:4, 6, n_sls), (1:4) or (1:4, 6), in the group layout
+        const int k = x % 4, v = x / 4;
+        const GroupMeta &g = h->os.group(s);
+        const int ge = (int)(s - g.slot0);
+        if (field == AXG_FIELD_MEMVAR) at = cg_state_at(g, ge, k, v / 6, v % 6, nsls);
+        else at = cg_state_at(g, ge, k, nsls, field == AXG_FIELD_ATT_SRC_TR ? 6 : v, nsls);
+      }
+      if (out) out[e * len + x] = st[at];
+      else st[at] = in[e * len + x];
+    }
   }
   if (in) {
-    CK(cudaMemcpyAsync(h->an.state, st.data(), st.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(dev, st.data(), st.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
   }
   return AXG_OK;
@@ -1997,8 +2099,9 @@ int axg_reset(axg_handle *h) {
   // the iter-0 seismogram sample (dump_stuff(0,...)) is the zero wavefield
   CK(cudaMemsetAsync(h->rec, 0, (size_t)h->nseismo * 3 * std::max(h->num_rec, 1) * sizeof(float), h->stream));
   CK(cudaMemsetAsync(h->iter, 0, 4 * sizeof(int32_t), h->stream));
-  if (h->anel || h->anel_full)
+  if (h->anel_full)
     CK(cudaMemsetAsync(h->an.state, 0, (size_t)h->nel_s * h->an.state_stride * sizeof(float), h->stream));
+  if (h->anel) CK(cudaMemsetAsync(h->cg.state, 0, (size_t)cg_floats(h) * sizeof(float), h->stream));
   for (float *p : {h->cu_s[0], h->cu_s[1], h->cu_s[2], h->cv_s[0], h->cv_s[1], h->cv_s[2], h->cu_f, h->cv_f})
     if (p) CK(cudaMemsetAsync(p, 0, (p == h->cu_f || p == h->cv_f ? h->nglob_f : h->nglob_s) * sizeof(float), h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -2103,7 +2206,7 @@ unsigned gvec_grid(const axg_handle *h, int64_t n) {
 int gvec_io_prepare(axg_handle *h) {
   if (h->gvec_perm) return AXG_OK;
   int rc;
-  if ((rc = upload(h, &h->gvec_perm, h->ps.new_of_old))) return rc;
+  if ((rc = upload(h, &h->gvec_perm, h->os.new_of_old))) return rc;
   if ((rc = dalloc(h, &h->gvec_stage, 3 * (size_t)h->nglob_s))) return rc;
   if (!h->copy_stream) CK(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
   for (cudaEvent_t &e : h->ev_io) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -2506,7 +2609,8 @@ int axg_autotune(axg_handle *h, int32_t *chosen) {
     add(h->cu_s[c], gs), add(h->cv_s[c], gs);
   }
   add(h->fu, gf), add(h->fv, gf), add(h->fa, gf), add(h->ff, gf), add(h->cu_f, gf), add(h->cv_f, gf);
-  if (h->anel || h->anel_full) add(h->an.state, (size_t)h->nel_s * h->an.state_stride * sizeof(float));
+  if (h->anel_full) add(h->an.state, (size_t)h->nel_s * h->an.state_stride * sizeof(float));
+  if (h->anel) add(h->cg.state, (size_t)cg_floats(h) * sizeof(float));
   add(h->rec, (size_t)h->nseismo * 3 * std::max(h->num_rec, 1) * sizeof(float));
   add(h->iter, 4 * sizeof(int32_t));
   size_t total = 0;
@@ -2588,12 +2692,16 @@ int axg_set_compensated(axg_handle *h, int32_t on) {
     const bool mono = h->pole == AXG_MONOPOLE;
     for (int c = 0; c < 3; ++c) {
       if (mono && c == 1) continue;
-      if ((rc = dalloc(h, &h->cu_s[c], h->nglob_s)) || (rc = dalloc(h, &h->cv_s[c], h->nglob_s))) return rc;
+      if ((rc = dalloc(h, &h->cu_s[c], h->nglob_s)) || (rc = dalloc(h, &h->cv_s[c], h->nglob_s)) ||
+          (rc = dalloc(h, &h->cup_s[c], h->nglob_s)))
+        return rc;
       CK(cudaMemsetAsync(h->cu_s[c], 0, h->nglob_s * sizeof(float), h->stream));
       CK(cudaMemsetAsync(h->cv_s[c], 0, h->nglob_s * sizeof(float), h->stream));
     }
     if (h->nel_f > 0) {
-      if ((rc = dalloc(h, &h->cu_f, h->nglob_f)) || (rc = dalloc(h, &h->cv_f, h->nglob_f))) return rc;
+      if ((rc = dalloc(h, &h->cu_f, h->nglob_f)) || (rc = dalloc(h, &h->cv_f, h->nglob_f)) ||
+          (rc = dalloc(h, &h->cup_f, h->nglob_f)))
+        return rc;
       CK(cudaMemsetAsync(h->cu_f, 0, h->nglob_f * sizeof(float), h->stream));
       CK(cudaMemsetAsync(h->cv_f, 0, h->nglob_f * sizeof(float), h->stream));
     }
@@ -2635,13 +2743,13 @@ int axg_set_time_scheme(axg_handle *h, int32_t scheme, const float *stf_stages) 
                   "symplectic schemes: a fluid source and a fluid free surface are not supported (the reference's "
                   "symplectic loop applies neither)");
     if (!stf_stages) return fail(h, AXG_ERR_BAD_ARG, "stf_stages is NULL");
-    if (h->anel_full)
-      return fail(h, AXG_ERR_UNSUPPORTED,
-                  "symplectic schemes with attenuation at every GLL point (att_coarse_grained = 0) are not supported");
-    if (h->anel) {  // per launch slot: the element's points and axis flag
+    if (h->anel) {  // the memory variables' update visits each slot's points
       const int rc = upload_slot_points(h);
       if (rc) return rc;
     }
+    if (h->anel_full)
+      return fail(h, AXG_ERR_UNSUPPORTED,
+                  "symplectic schemes with attenuation at every GLL point (att_coarse_grained = 0) are not supported");
     h->sym_cd.resize(n + 1);
     h->sym_cv.resize(n);
     for (int i = 0; i <= n; ++i) h->sym_cd[i] = cd[i] * h->dt;
@@ -2655,13 +2763,7 @@ int axg_set_time_scheme(axg_handle *h, int32_t scheme, const float *stf_stages) 
   drop_graphs(h);
   int rc = prepare_kernels(h);
   if (rc) return rc;
-  if (h->scheme) {
-    h->kernels_per_step = (int64_t)h->nstages * (h->ps.n_colours + (h->nel_f > 0 ? 2 +
-                          (h->to_fluid.n > 0) + (h->to_solid.n > 0) : 0)) + 2 + (h->anel ? 1 : 0);
-  } else {
-    h->kernels_per_step = h->ps.n_colours + 1 + (h->anel_full ? 1 : 0) +
-                          (h->nel_f > 0 ? 2 + (h->to_fluid.n > 0) + (h->to_solid.n > 0) : 0);
-  }
+  count_launches(h);
   return axg_reset(h);
 }
 
@@ -2685,8 +2787,8 @@ int axg_get_info(axg_handle *h, axg_info *info) {
   info->growth_fluid = h->pf.growth;
   info->steps_per_graph = h->steps_per_graph;
   info->mesh_bytes = h->mesh ? h->mesh->bytes : 0;
-  info->ctas_per_sm_force = h->solid_ctas / std::max(h->num_sms, 1);
-  info->ctas_per_sm_step = h->solid_ctas_step / std::max(h->num_sms, 1);
+  info->ctas_per_sm_force = h->elem_ctas_force;
+  info->ctas_per_sm_step = h->elem_ctas_step;
   return AXG_OK;
 }
 
@@ -2765,7 +2867,11 @@ void axg_destroy(axg_handle *h) {
 int axg_device_check_report(int32_t *out8) {
   if (!out8) return fail(nullptr, AXG_ERR_BAD_ARG, "out8 is NULL");
 #ifdef AXG_DEVICE_CHECKS
+  // one record per translation unit of kernels: the first that holds a violation
   cudaError_t e = cudaMemcpyFromSymbol(out8, g_axg_check, 8 * sizeof(int32_t));
+  if (e == cudaSuccess && !out8[0]) e = stream_check_record<POLE_MONO>(out8);
+  if (e == cudaSuccess && !out8[0]) e = stream_check_record<POLE_DI>(out8);
+  if (e == cudaSuccess && !out8[0]) e = stream_check_record<POLE_QUAD>(out8);
   if (e != cudaSuccess) return fail(nullptr, AXG_ERR_CUDA, cudaGetErrorString(e));
   return AXG_OK;
 #else
@@ -2953,8 +3059,6 @@ struct axg_batch {
   std::vector<axg_handle *> hs;
   int device = 0, num_sms = 1;
   SpecDev spec{};
-  // resident CTAs of the batched solid kernels per (symplectic, pole, compensated, attenuated)
-  int solid_ctas[2][3][2][2] = {};
   cudaStream_t stream = nullptr;
   // one step of every solve, captured with the plain Newmark solves' buffer
   // roles at parity 0 and at parity 1 (trade_buffers); steps alternate them
@@ -3020,142 +3124,47 @@ void stage_states(axg_handle *h, int stage, StateArgs &ss, StateArgs &fs) {
   }
 }
 
-// the fluid's two passes for the solves of a phase, per class (non-monopole, compensated)
-template <int NONMONO, bool KAHAN>
-int64_t batch_fluid(axg_batch *b, int stage, cudaStream_t s) {
-  auto mine = [&](axg_handle *h) {
-    return in_stage(h, stage) && h->nel_f > 0 && (h->pole != AXG_MONOPOLE) == (NONMONO != 0) && h->kahan == KAHAN;
-  };
-  auto work = [&](axg_handle *h) {
-    FluidArgs fa = fluid_args(h);
-    if (stage >= 0) fa.fsmask = nullptr;  // symplectic_time_loop applies no free-surface mask
-    StateArgs ss, fs;
-    stage_states(h, stage, ss, fs);
-    return FluidWork{fa, fs};
-  };
-  const int64_t ne = for_batches<FluidWork>(
-      b->hs, [&](axg_handle *h) { return mine(h) ? (int32_t)h->nel_f : 0; }, work,
-      [&](const Many<FluidWork> &m) {
-        const unsigned g = fluid_elem_grid(m.start[m.n]);
-        if (stage < 0)
-          fluid_elem_kernel<NONMONO, MODE_NEWMARK, KAHAN, Many<FluidWork>><<<g, kFlElemThreads, 0, s>>>(m, b->spec);
-        else
-          fluid_elem_kernel<NONMONO, MODE_SYMPLECTIC, KAHAN, Many<FluidWork>><<<g, kFlElemThreads, 0, s>>>(m, b->spec);
-      });
-  const int64_t np = for_batches<FluidWork>(
-      b->hs, [&](axg_handle *h) { return mine(h) ? (int32_t)h->nglob_f : 0; }, work,
-      [&](const Many<FluidWork> &m) {
-        const unsigned g = (unsigned)((m.start[m.n] + 255) / 256);
-        if (stage < 0) fluid_point_kernel<NONMONO, MODE_NEWMARK, KAHAN, Many<FluidWork>><<<g, 256, 0, s>>>(m);
-        else fluid_point_kernel<NONMONO, MODE_SYMPLECTIC, KAHAN, Many<FluidWork>><<<g, 256, 0, s>>>(m);
-      });
-  return ne + np;
-}
-
-// a solve's colour work with its attenuation data (attenuated batches)
-struct AnelPatchWork {
-  PatchWork pw;
-  AnelArgs an;
-};
-
-template <int POLE, int MODE, bool KAHAN, bool ANEL>
-int64_t batch_solid_colour(axg_batch *b, int stage, int c, cudaStream_t s) {
-  const int pole = POLE == POLE_MONO ? AXG_MONOPOLE : POLE == POLE_DI ? AXG_DIPOLE : AXG_QUADPOLE;
-  return for_batches<AnelPatchWork>(
-      b->hs,
-      [&](axg_handle *h) {
-        const bool mine = in_stage(h, stage) && c < h->ps.n_colours && h->pole == pole && h->kahan == KAHAN &&
-                          h->anel == ANEL;
-        return mine ? h->ps.colour_start[c + 1] - h->ps.colour_start[c] : 0;
-      },
-      [&](axg_handle *h) {
-        DomainArgs a = domain_args(h->ds, h->ps);
-        a.patch_begin = h->ps.colour_start[c];
-        StateArgs ss, fs;
-        stage_states(h, stage, ss, fs);
-        return AnelPatchWork{PatchWork{a, ss}, h->an};
-      },
-      [&](const Many<AnelPatchWork> &mw) {
-        Many<PatchWork> m{};
-        m.n = mw.n;
-        std::memcpy(m.start, mw.start, sizeof(m.start));
-        for (int q = 0; q < mw.n; ++q) m.w[q] = mw.w[q].pw;
-        const int grid = std::min(m.start[m.n], b->solid_ctas[MODE == MODE_SYMPLECTIC][POLE][KAHAN][ANEL]);
-        constexpr int smem = solid_smem_bytes<POLE, MODE, ANEL, KAHAN>();
-        if constexpr (ANEL) {
-          AnelBatch an{};
-          for (int q = 0; q < mw.n; ++q) an.a[q] = mw.w[q].an;
-          solid_anel_batch_kernel<POLE, MODE, KAHAN><<<grid, kThreads, smem, s>>>(m, b->spec, an);
-        } else {
-          solid_batch_kernel<POLE, MODE, KAHAN><<<grid, kThreads, smem, s>>>(m, b->spec);
-        }
-      });
-}
-
-// colour c of the solid, every pole and precision mode, plain and attenuated
-template <int MODE>
-int64_t batch_solid_colours(axg_batch *b, int stage, int c, cudaStream_t s) {
-  return batch_solid_colour<POLE_MONO, MODE, false, false>(b, stage, c, s) +
-         batch_solid_colour<POLE_MONO, MODE, true, false>(b, stage, c, s) +
-         batch_solid_colour<POLE_DI, MODE, false, false>(b, stage, c, s) +
-         batch_solid_colour<POLE_DI, MODE, true, false>(b, stage, c, s) +
-         batch_solid_colour<POLE_QUAD, MODE, false, false>(b, stage, c, s) +
-         batch_solid_colour<POLE_QUAD, MODE, true, false>(b, stage, c, s) +
-         batch_solid_colour<POLE_MONO, MODE, false, true>(b, stage, c, s) +
-         batch_solid_colour<POLE_MONO, MODE, true, true>(b, stage, c, s) +
-         batch_solid_colour<POLE_DI, MODE, false, true>(b, stage, c, s) +
-         batch_solid_colour<POLE_DI, MODE, true, true>(b, stage, c, s) +
-         batch_solid_colour<POLE_QUAD, MODE, false, true>(b, stage, c, s) +
-         batch_solid_colour<POLE_QUAD, MODE, true, true>(b, stage, c, s);
-}
-
-template <int POLE>
-int64_t batch_to_solid(axg_batch *b, int stage, cudaStream_t s) {
-  const int pole = POLE == POLE_MONO ? AXG_MONOPOLE : POLE == POLE_DI ? AXG_DIPOLE : AXG_QUADPOLE;
-  return for_batches<ToSolidWork>(
-      b->hs,
-      [&](axg_handle *h) { return in_stage(h, stage) && h->nel_f > 0 && h->pole == pole ? h->to_solid.n : 0; },
-      [&](axg_handle *h) {
-        StateArgs ss, fs;
-        stage_states(h, stage, ss, fs);
-        return ToSolidWork{h->to_solid, fs, ss};
-      },
-      [&](const Many<ToSolidWork> &m) {
-        couple_to_solid_kernel<POLE, Many<ToSolidWork>><<<(m.start[m.n] + 255) / 256, 256, 0, s>>>(m);
-      });
-}
-
-template <int DIPOLE>
-int64_t batch_to_fluid(axg_batch *b, int stage, cudaStream_t s) {
-  return for_batches<ToFluidWork>(
-      b->hs,
-      [&](axg_handle *h) {
-        return in_stage(h, stage) && h->nel_f > 0 && (h->pole == AXG_DIPOLE) == (DIPOLE != 0) ? h->to_fluid.n : 0;
-      },
-      [&](axg_handle *h) {
-        StateArgs ss, fs;
-        stage_states(h, stage, ss, fs);
-        return ToFluidWork{h->to_fluid, ss, h->ff, h->ds.axmask};
-      },
-      [&](const Many<ToFluidWork> &m) {
-        couple_to_fluid_kernel<DIPOLE, Many<ToFluidWork>><<<(m.start[m.n] + 255) / 256, 256, 0, s>>>(m);
-      });
-}
-
-// One phase of the solves taking part in it, in the order of enqueue_step
-// (enqueue_step_symplectic for a stage): coupling into the fluid, fluid
-// colours, coupling into the solid, solid colours.
-template <int MODE>
+// One phase of the solves taking part in it, as enqueue_step (a stage of
+// enqueue_step_symplectic) queues it for one: launch q of every solve of a
+// class (pole, form of the element pass, precision mode, attenuation) in one
+// launch.
 int64_t enqueue_batch_phase(axg_batch *b, int stage, cudaStream_t s) {
-  int64_t nl = batch_to_fluid<0>(b, stage, s) + batch_to_fluid<1>(b, stage, s);
-  int sc = 0;
-  for (axg_handle *h : b->hs)
-    if (in_stage(h, stage)) sc = std::max(sc, h->ps.n_colours);
-  nl += batch_fluid<0, false>(b, stage, s) + batch_fluid<0, true>(b, stage, s) + batch_fluid<1, false>(b, stage, s) +
-        batch_fluid<1, true>(b, stage, s);
-  nl += batch_to_solid<POLE_MONO>(b, stage, s) + batch_to_solid<POLE_DI>(b, stage, s) +
-        batch_to_solid<POLE_QUAD>(b, stage, s);
-  for (int c = 0; c < sc; ++c) nl += batch_solid_colours<MODE>(b, stage, c, s);
+  const int mode = stage < 0 ? MODE_NEWMARK : MODE_SYMPLECTIC;
+  int64_t nl = 0;
+  for (int cls = 0; cls < 24; ++cls) {
+    const int pole = cls / 8;
+    const bool kahan = cls & 1, anel = (cls & 2) != 0, patched = (cls & 4) != 0;
+    // per launch of the class: its kind and the solves' work
+    std::vector<std::pair<int, std::vector<StreamWork>>> seq;
+    for (axg_handle *h : b->hs) {
+      if (!in_stage(h, stage) || h->pole != pole || h->kahan != kahan || h->anel != anel ||
+          h->os.patched != patched)
+        continue;
+      StateArgs ss, fs;
+      stage_states(h, stage, ss, fs);
+      size_t q = 0;
+      stream_launches(h, mode, stream_work(h, mode, ss, fs), [&](int kind, const StreamWork &w) {
+        // the next launch of the same kind (a solve may need fewer of either)
+        while (q < seq.size() && seq[q].first != kind) ++q;
+        if (q == seq.size()) seq.emplace_back(kind, std::vector<StreamWork>());
+        seq[q++].second.push_back(w);
+      });
+    }
+    for (auto &l : seq)
+      for (size_t k0 = 0; k0 < l.second.size(); k0 += kMaxStream) {
+        StreamMany m{};
+        for (size_t k = k0; k < l.second.size() && m.n < kMaxStream; ++k) {
+          m.w[m.n] = l.second[k];
+          m.start[m.n + 1] = m.start[m.n] + stream_blocks(l.second[k]);
+          ++m.n;
+        }
+        const StreamKernel k{l.first, mode, patched, anel, kahan};
+        if (pole == AXG_MONOPOLE) stream_launch<POLE_MONO>(k, m, b->spec, s);
+        else if (pole == AXG_DIPOLE) stream_launch<POLE_DI>(k, m, b->spec, s);
+        else stream_launch<POLE_QUAD>(k, m, b->spec, s);
+        ++nl;
+      }
+  }
   return nl;
 }
 
@@ -3163,11 +3172,11 @@ int64_t enqueue_batch_phase(axg_batch *b, int stage, cudaStream_t s) {
 // stages (stage i of every solve with more than i stages in one phase), their
 // final drifts and memory variables, then the seismograms and step counters.
 int64_t enqueue_batch_step(axg_batch *b, cudaStream_t s) {
-  int64_t nl = enqueue_batch_phase<MODE_NEWMARK>(b, -1, s);
-  for (axg_handle *h : b->hs) trade_buffers(h);  // the plain Newmark solves' state after the step
+  int64_t nl = enqueue_batch_phase(b, -1, s);
+  for (axg_handle *h : b->hs) trade_buffers(h);  // the Newmark solves' state after the step
   int ns = 0;
   for (axg_handle *h : b->hs) ns = std::max(ns, h->scheme != AXG_SCHEME_NEWMARK2 ? h->nstages : 0);
-  for (int i = 0; i < ns; ++i) nl += enqueue_batch_phase<MODE_SYMPLECTIC>(b, i, s);
+  for (int i = 0; i < ns; ++i) nl += enqueue_batch_phase(b, i, s);
   if (ns > 0) {
     nl += for_batches<DriftWork>(
         b->hs, [](axg_handle *h) { return h->scheme != AXG_SCHEME_NEWMARK2 ? drift_points(h) : 0; },
@@ -3175,21 +3184,21 @@ int64_t enqueue_batch_step(axg_batch *b, cudaStream_t s) {
         [&](const Many<DriftWork> &m) { drift_kernel<Many<DriftWork>><<<(m.start[m.n] + 255) / 256, 256, 0, s>>>(m); });
     for (axg_handle *h : b->hs)
       if (h->scheme != AXG_SCHEME_NEWMARK2 && h->anel) {
-        launch_anel_memvar_pole(h, s);
+        launch_anel_memvar(h, s);
         ++nl;
       }
   }
+  // (a Newmark solve's last launch records its seismograms)
   nl += for_batches<RecWork>(
-      b->hs, [](axg_handle *) { return 1; }, [](axg_handle *h) { return rec_work(h, solid_state(h)); },
+      b->hs, [](axg_handle *h) { return h->scheme != AXG_SCHEME_NEWMARK2 ? 1 : 0; },
+      [](axg_handle *h) { return rec_work(h, solid_state(h)); },
       [&](const Many<RecWork> &m) { receivers_kernel<Many<RecWork>><<<m.n, 256, 0, s>>>(m); });
   return nl;
 }
 
 // kernel parameters are limited to 32764 bytes
-static_assert(sizeof(Many<PatchWork>) + sizeof(SpecDev) + sizeof(AnelBatch) <= 32000 &&
-                  sizeof(Many<FluidWork>) + sizeof(SpecDev) <= 32000 &&
-                  sizeof(Many<ToSolidWork>) <= 32000 && sizeof(Many<DriftWork>) <= 32000 &&
-                  sizeof(Many<ToFluidWork>) <= 32000 && sizeof(Many<RecWork>) <= 32000,
+static_assert(sizeof(StreamMany) + sizeof(SpecDev) <= 32000 && sizeof(Many<DriftWork>) <= 32000 &&
+                  sizeof(Many<RecWork>) <= 32000,
               "a batched launch's descriptors must fit the kernel parameter space");
 
 // the step counters of up to kMaxBatch solves
@@ -3200,32 +3209,6 @@ struct IterSet {
 };
 __global__ void set_iters_kernel(const __grid_constant__ IterSet a) {
   if ((int)threadIdx.x < a.n) *a.ctr[threadIdx.x] = a.first[threadIdx.x];
-}
-
-template <int POLE, int MODE, bool KAHAN, bool ANEL>
-int prepare_batch_kernel(axg_batch *b, axg_handle *h) {
-  int *ctas = &b->solid_ctas[MODE == MODE_SYMPLECTIC][POLE][KAHAN][ANEL];
-  constexpr int smem = solid_smem_bytes<POLE, MODE, ANEL, KAHAN>();
-  int rc;
-  if constexpr (ANEL) rc = prepare_kernel_fn(h, solid_anel_batch_kernel<POLE, MODE, KAHAN>, smem, ctas);
-  else rc = prepare_kernel_fn(h, solid_batch_kernel<POLE, MODE, KAHAN>, smem, ctas);
-  if (rc) b->err = h->err;
-  return rc;
-}
-
-template <int POLE, int MODE>
-int prepare_batch_kernels(axg_batch *b, axg_handle *h) {
-  if (h->anel)
-    return h->kahan ? prepare_batch_kernel<POLE, MODE, true, true>(b, h) : prepare_batch_kernel<POLE, MODE, false, true>(b, h);
-  return h->kahan ? prepare_batch_kernel<POLE, MODE, true, false>(b, h) : prepare_batch_kernel<POLE, MODE, false, false>(b, h);
-}
-
-// the batched solid kernel a solve of the batch launches
-template <int MODE>
-int prepare_batch_mode(axg_batch *b, axg_handle *h) {
-  if (h->pole == AXG_MONOPOLE) return prepare_batch_kernels<POLE_MONO, MODE>(b, h);
-  if (h->pole == AXG_DIPOLE) return prepare_batch_kernels<POLE_DI, MODE>(b, h);
-  return prepare_batch_kernels<POLE_QUAD, MODE>(b, h);
 }
 
 int batch_create_impl(axg_batch *b, axg_handle *const *hs, int32_t n) {
@@ -3252,11 +3235,6 @@ int batch_create_impl(axg_batch *b, axg_handle *const *hs, int32_t n) {
   b->device = hs[0]->device;
   b->spec = hs[0]->spec;
   b->num_sms = hs[0]->num_sms;
-  for (axg_handle *h : b->hs) {
-    const int rc = h->scheme == AXG_SCHEME_NEWMARK2 ? prepare_batch_mode<MODE_NEWMARK>(b, h)
-                                                    : prepare_batch_mode<MODE_SYMPLECTIC>(b, h);
-    if (rc) return rc;
-  }
   BCK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   BCK(cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming));
   // the solves' buffers in their parity-0 roles (each solve's stream is idle)

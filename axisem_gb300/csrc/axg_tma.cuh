@@ -116,7 +116,7 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // Bounded wait for the phase of `bar` with `parity`; returns false when it
 // gave up, after recording AXG_ERR_TIMEOUT in *err.  The first poll is the
 // fast path; the timer is read only once the wait is pending.
-__device__ __noinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, int32_t *err) {
+static __device__ __noinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, int32_t *err) {
   const uint64_t t0 = globaltimer_ns();
   bool checked = false;
   for (;;) {

@@ -1,0 +1,78 @@
+"""GPU tests of the two forms of the solid's element pass: scattered (a buffer
+of element contributions, summed per point) and patched (large meshes:
+accumulated in shared memory, own points finished by the patch).
+
+Sizes are where they can go wrong: solids of fewer elements than a group of
+six, of group and CTA remainders, with every element on the axis; a patched
+solid of ragged patches, with coupled points and the source inside patches and
+on their edges.  Tolerance: relative L2 <= 1e-5 against the FP64 oracle for
+the stiffness, 1e-4 for wavefields after a few steps, the bars of the other
+parity tests (FP32 sums of some tens of terms in another order)."""
+import numpy as np
+import pytest
+
+from axisem_gb300 import _abi
+from axisem_gb300.mesh import coupled_mesh, gauss_at, gvec_to_elemental, random_gvec, structured_mesh
+from axisem_gb300.solver import Solver, symplectic_coefficients
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.linalg.norm(np.asarray(a, np.float64) - b) / max(np.linalg.norm(b), 1e-300))
+
+
+@pytest.mark.parametrize("pole", [0, 1, 2])
+@pytest.mark.parametrize("ni,nj,axial", [(1, 1, "none"), (1, 1, "column"), (5, 1, "none"), (1, 7, "column"),
+                                         (3, 4, "random1pct"), (5, 5, "column"), (13, 1, "random1pct")])
+def test_group_remainders(gpu_lib, orc, pole, ni, nj, axial):
+    m = structured_mesh(ni, nj, pole, axial=axial, seed=3)
+    u = random_gvec(m, seed=4)
+    with Solver(m) as s:
+        f = s.stiffness_assembled(u)
+        assert np.array_equal(f, s.stiffness_assembled(u))
+    assert rel(f, orc.stiffness_assembled(m, u, np.float64)) <= 1e-5
+
+
+PATCHED = (367, 359)   # 131 753 elements: patched; not multiples of a patch's 8 x 8
+
+
+@pytest.mark.parametrize("pole", [0, 1, 2])
+def test_patched_stiffness(gpu_lib, orc, pole):
+    m = structured_mesh(*PATCHED, pole, terms="pole", axial="random1pct", seed=11)
+    u = random_gvec(m, seed=12)
+    with Solver(m) as s:
+        f = s.stiffness_assembled(u)
+        assert np.array_equal(f, s.stiffness_assembled(u))
+    assert rel(f, orc.stiffness_assembled(m, u, np.float64)) <= 1e-5
+
+
+@pytest.mark.parametrize("pole,mode,absorbing", [(0, "plain", True), (1, "plain", False), (2, "comp", False),
+                                                 (1, "comp", True), (2, "symplec4", False)])
+def test_patched_steps(gpu_lib, orc, pole, mode, absorbing):
+    """From a random displacement, so that every patch takes part."""
+    n = 6
+    m = coupled_mesh(PATCHED[0], PATCHED[1], 9, pole, niter=n, num_rec=9, seis_it=1, terms="pole", absorbing=absorbing,
+                     src_row=8 if pole == 1 else 11)
+    u = random_gvec(m, seed=5)
+    if pole == 0:
+        u[:, 1] = 0.0
+    t = orc.TimeLoop(m, np.float64)
+    t.disp[...] = gvec_to_elemental(m, u)
+    with Solver(m) as s:
+        s.set_compensated(mode == "comp")
+        if mode == "symplec4":
+            _, _, coeff = symplectic_coefficients(_abi.SCHEME_SYMPLEC4, m.deltat)
+            stf = gauss_at(np.arange(n)[:, None] * m.deltat + coeff[None, :], 20 * m.deltat)
+            s.set_time_scheme(_abi.SCHEME_SYMPLEC4, stf)
+            assert t.run_symplectic(1, n, _abi.SCHEME_SYMPLEC4, stf) == 0
+        else:
+            assert t.run(1, n) == 0
+        s.upload_disp(u)
+        s.run(1, 4)
+        s.run(5, 2)
+        comps = [0, 2] if pole == 0 else [0, 1, 2]
+        assert rel(s.receivers()[1:], t.receivers()[1:]) <= 1e-4
+        assert rel(s.get_state(_abi.FIELD_DISP)[..., comps], t.disp[..., comps]) <= 1e-4
+        assert rel(s.get_state(_abi.FIELD_VELO)[..., comps], t.velo[..., comps]) <= 1e-4
+        assert rel(s.get_state(_abi.FIELD_CHI), t.chi) <= 1e-4
