@@ -1071,10 +1071,11 @@ struct SolidPoint {
     }
   }
 
-  // the source term of point g, if it has one
-  static __device__ __forceinline__ void source(const StreamWork &w, int64_t g, float (&sum)[NC]) {
-    const StateArgs &st = w.solid;
-    const float stf1 = AXG_BOUND(*w.iter_p - 1, st.niter, 66) ? st.stf[*w.iter_p - 1] : 0.f;
+  // the source term of point g, if it has one, in step `iter` (the element
+  // pass reads the step counter, the point pass the copy the element pass
+  // makes of it: each pass writes the other's)
+  static __device__ __forceinline__ void source(const StateArgs &st, int32_t iter, int64_t g, float (&sum)[NC]) {
+    const float stf1 = AXG_BOUND(iter - 1, st.niter, 66) ? st.stf[iter - 1] : 0.f;
     if (stf1 == 0.f) return;
     for (int q = 0; q < st.src.n; ++q)
       if (st.src.gidx[q] == (int32_t)g) {
@@ -1186,7 +1187,7 @@ __device__ __forceinline__ void solid_point(const StreamWork &w, int64_t g) {
     return;
   }
   if (stopped) return;  // a stopped solve does nothing more
-  if (s0 & kStSource) S::source(w, g, sum);
+  if (s0 & kStSource) S::source(st, *w.iter_p, g, sum);
   pt.finish(st, g, (s0 & kStAxis) != 0, sum);
 }
 
@@ -1346,7 +1347,7 @@ __device__ __forceinline__ void patch_cta(const StreamWork &w, const SpecDev &sp
 #pragma unroll
         for (int c = 0; c < NC; ++c) st.f[S::gc(c)][g] = sum[c];
       } else {
-        if (src) S::source(w, g, sum);
+        if (src) S::source(st, *st.iter, g, sum);
         pt[b].finish(st, g, ax[b] != 0, sum);
       }
     }
