@@ -175,6 +175,10 @@ struct axg_handle {
   int graph_steps[2] = {};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t ev_done = nullptr;  // end of the work axg_run_async queued
+  // axg_run: the flags after each graph (page-locked, made on first use), and
+  // when they have landed; two graphs are queued at a time
+  int32_t *run_flags = nullptr;
+  cudaEvent_t ev_flags[2] = {};
   bool pending = false;
   int num_sms = 1;
   int elem_ctas_force = 1, elem_ctas_step = 1;  // resident CTAs per SM of the element pass
@@ -1185,6 +1189,9 @@ void release(axg_handle *h) {
   if (h->ev_done) cudaEventDestroy(h->ev_done);
   for (cudaEvent_t e : h->ev_io)
     if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : h->ev_flags)
+    if (e) cudaEventDestroy(e);
+  if (h->run_flags) cudaFreeHost(h->run_flags);
   for (int k = 0; k < 2; ++k) {
     if (h->dump.ev_dump[k]) cudaEventDestroy(h->dump.ev_dump[k]);
     if (h->dump.ev_copy[k]) cudaEventDestroy(h->dump.ev_copy[k]);
@@ -2118,30 +2125,43 @@ int axg_run(axg_handle *h, int32_t first_iter, int32_t n_iter) {
     int rc = axg_run_async(h, first_iter, n_iter);
     return rc ? rc : axg_wait(h);
   }
+  if (!h->run_flags) {
+    CK(cudaHostAlloc((void **)&h->run_flags, 4 * sizeof(int32_t), cudaHostAllocDefault));
+    for (cudaEvent_t &e : h->ev_flags) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
   CK(cudaMemcpyAsync(h->iter, &first_iter, sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
   CK(refresh_predicted(h, h->stream));
-  int32_t done = 0;
-  while (done < n_iter) {
+  // Graph q + 1 is queued before the flags of graph q are waited for, so that
+  // the device does not idle while the host polls (a stopped solve's kernels
+  // return at once).  Polling each graph before the next had cost 10 us per
+  // graph: 3.66 against 3.40 ms for 400 steps of the PREM 50 s mesh.
+  auto poll = [&](int q) -> int {
+    CK(cudaEventSynchronize(h->ev_flags[q & 1]));
+    const int32_t *f = h->run_flags + 2 * (q & 1);
+    if (f[1] != 0) return fail(h, AXG_ERR_TIMEOUT, "a bounded device wait gave up");
+    if (f[0] != 0)
+      return fail(h, AXG_ERR_BLOWUP,
+                  fmt("displacements blew up: |disp(1,1,:,:)| > 10 |magnitude| at time step %d", f[0] + 1));
+    return AXG_OK;
+  };
+  int rc = AXG_OK, q = 0;
+  for (int32_t done = 0; done < n_iter && rc == AXG_OK; ++q) {
     const int k = std::min<int32_t>(h->steps_per_graph, n_iter - done);
     if (k == h->steps_per_graph) {
-      const int rc = launch_graph(h, k, h->graph, h->graph_steps);
-      if (rc) return rc;
+      if ((rc = launch_graph(h, k, h->graph, h->graph_steps))) break;
     } else {
       for (int s = 0; s < k; ++s) enqueue_step(h, h->stream);
       CK(cudaGetLastError());
     }
     done += k;
-    int32_t flags[2] = {0, 0};
-    CK(cudaMemcpyAsync(flags, h->blowup, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    const int32_t bl = flags[0];
-    if (flags[1] != 0)
-      return fail(h, AXG_ERR_TIMEOUT, "a bounded device wait on a bulk copy gave up");
-    if (bl != 0)
-      return fail(h, AXG_ERR_BLOWUP,
-                  fmt("displacements blew up: |disp(1,1,:,:)| > 10 |magnitude| at time step %d", bl + 1));
+    CK(cudaMemcpyAsync(h->run_flags + 2 * (q & 1), h->blowup, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaEventRecord(h->ev_flags[q & 1], h->stream));
+    if (q > 0) rc = poll(q - 1);
   }
-  return AXG_OK;
+  if (rc == AXG_OK && q > 0) rc = poll(q - 1);
+  // the run is complete, also where it stopped early
+  if (rc != AXG_OK && rc != AXG_ERR_CUDA) CK(cudaStreamSynchronize(h->stream));
+  return rc;
 }
 
 }  // extern "C"
