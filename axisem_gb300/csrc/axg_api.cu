@@ -98,6 +98,7 @@ struct StreamOrder {
   std::vector<int32_t> new_of_old, old_of_new;  // point numbering
   std::vector<GroupMeta> groups;
   std::vector<int32_t> group_of_slot;
+  int64_t n_off = 0;                            // scattered: elements off the axis, before the axial ones
   int64_t n_own = 0;
   std::vector<PatchInfo> patches;
   std::vector<int32_t> def;                     // deferred points, patch by patch (internal numbers)
@@ -446,12 +447,12 @@ void parallel_ranges(int64_t n, Fn fn) {
 
 // The order of a domain: elements patch by patch in creation order
 // (neighbouring groups then share points, which stay in L1 and L2).
-// Scattered: those of a patch in the reference's order, `last` elements (the
-// fluid's axial ones) at the end, groups of six across patches; points by the
+// Scattered: those of a patch in the reference's order, the axial elements at
+// the end, groups of six across patches (`split`: of either kind); points by the
 // first and second patch that hold them.  Patched: those of a patch round by
 // round (the elements of a round share no point), groups within a round.
 void stream_order(const DomainPlan &pl, const int32_t *igloc, const std::vector<uint8_t> &coupled,
-                  const std::vector<uint8_t> *last, bool patched, StreamOrder &o) {
+                  const std::vector<uint8_t> &axial, bool patched, bool split, StreamOrder &o) {
   const int64_t nel = pl.nel, nglob = pl.nglob;
   const int32_t np = pl.n_patches;
   o = StreamOrder();
@@ -489,9 +490,11 @@ void stream_order(const DomainPlan &pl, const int32_t *igloc, const std::vector<
     for (int64_t e = 0; e < nel; ++e) fill[pl.patch_of_elem[e] + 1]++;
     for (int32_t p = 0; p < np; ++p) fill[p + 1] += fill[p];
     for (int64_t e = 0; e < nel; ++e) o.elem_order[fill[pl.patch_of_elem[e]]++] = (int32_t)e;
-    if (last)
-      std::stable_partition(o.elem_order.begin(), o.elem_order.end(), [&](int32_t e) { return !(*last)[e]; });
-    add_groups(0, nel, 0);
+    o.n_off = std::stable_partition(o.elem_order.begin(), o.elem_order.end(), [&](int32_t e) { return !axial[e]; }) -
+              o.elem_order.begin();
+    if (!split) o.n_off = nel;
+    add_groups(0, o.n_off, 0);
+    add_groups(o.n_off, nel, 0);
   }
   // the first and second patch of each point; a deferred point sorts after
   // every own point
@@ -973,6 +976,7 @@ StreamWork stream_work(axg_handle *h, int mode, const StateArgs &ss, const State
   StreamWork w{};
   w.ds = stream_domain(h->ds, h->nel_s, h->nglob_s);
   w.ds.aux = mode == MODE_NEWMARK && h->anel_full ? h->fx : nullptr;
+  w.ds.n_off = h->os.n_off;
   w.ds.n_patches = (int32_t)h->os.patches.size();
   w.ds.n_def = (int64_t)h->os.def.size();
   for (int32_t p : h->src_patches) w.ds.src_patch[w.ds.n_src_patch++] = p;
@@ -1011,7 +1015,7 @@ void stream_launches(const axg_handle *h, int mode, const StreamWork &base, Fn f
   const bool fluid = mode != MODE_FORCE && h->nel_f > 0;
   const int32_t nb_fp = fluid ? ceil_div(h->nglob_f, kGrpThreads) : 0;
   StreamWork w = base;
-  w.nb_se = h->os.patched ? (int32_t)h->os.patches.size() : ceil_div(grp_count(h->nel_s), kGrpWarps);
+  w.nb_se = h->os.patched ? (int32_t)h->os.patches.size() : ceil_div((int64_t)h->os.groups.size(), kGrpWarps);
   if (fluid) {
     w.nb_fe = ceil_div(grp_count(h->nel_f), kGrpWarps);
     w.nb_cp = ceil_div(h->to_fluid.n, kGrpThreads);
@@ -1618,10 +1622,11 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
     perr = validate_plan(h->igloc_s.data(), h->nel_s, h->nglob_s, h->pre_s, h->ps);
     if (!perr.empty()) return fail(h, AXG_ERR_BAD_DESC, "solid plan invalid: " + perr);
 #endif
-    stream_order(h->ps, h->igloc_s.data(), h->pre_s, nullptr, !h->anel && h->nel_s > kPatchedElems, h->os);
+    stream_order(h->ps, h->igloc_s.data(), h->pre_s, h->axial_s, !h->anel && h->nel_s > kPatchedElems,
+                 true, h->os);
     // the fluid's axial elements at the end, so that its warps seldom mix
     // axial and other elements
-    if (h->nel_f > 0) stream_order(h->pf, h->igloc_f.data(), h->pre_f, &h->axial_f, false, h->of);
+    if (h->nel_f > 0) stream_order(h->pf, h->igloc_f.data(), h->pre_f, h->axial_f, false, false, h->of);
     for (DomainPlan *p : {&h->ps, &h->pf}) {  // what only the patch kernel of the no-allocation entry point reads
       for (std::vector<int32_t> *v : {&p->elem_order, &p->new_of_old, &p->old_of_new}) std::vector<int32_t>().swap(*v);
       std::vector<uint32_t>().swap(p->pt_words);
