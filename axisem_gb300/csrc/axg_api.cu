@@ -159,6 +159,7 @@ struct axg_handle {
   float *inv_mass_s = nullptr, *inv_mass_f = nullptr, *gamma_s = nullptr, *gamma_f = nullptr;
   // FP64 inverse masses (mesh) and source values (solve), when the descriptor had them
   double *inv_mass_s_dp = nullptr, *inv_mass_f_dp = nullptr, *src_val_dp_d = nullptr;
+  float2 *inv_mass_s_pair = nullptr, *inv_mass_f_pair = nullptr;  // the same masses, where FP32 pairs hold them
   float *stf = nullptr, *rec = nullptr;
   int32_t *iter = nullptr, *blowup = nullptr, *rec_gidx_d = nullptr;
   int32_t *src_gidx_d = nullptr;
@@ -844,6 +845,7 @@ StateArgs solid_state(axg_handle *h) {
     s.cup[c] = h->kahan ? h->cup_s[c] : nullptr;
   }
   s.inv_mass = h->inv_mass_s;
+  s.inv_mass_pair = h->kahan ? h->inv_mass_s_pair : nullptr;
   s.inv_mass_dp = h->kahan ? h->inv_mass_s_dp : nullptr;
   s.gamma = h->gamma_s;
   s.stf = h->stf;
@@ -875,6 +877,7 @@ StateArgs fluid_state(axg_handle *h) {
   s.a[0] = h->fa;
   s.f[0] = h->ff;
   s.inv_mass = h->inv_mass_f;
+  s.inv_mass_pair = h->kahan ? h->inv_mass_f_pair : nullptr;
   s.inv_mass_dp = h->kahan ? h->inv_mass_f_dp : nullptr;
   s.gamma = h->gamma_f;
   s.src.n = 0;
@@ -1521,6 +1524,16 @@ void count_launches(axg_handle *h) {
   else h->kernels_per_step = h->nstages * count(MODE_SYMPLECTIC) + 2 + (h->anel ? 1 : 0);
 }
 
+// FP64 inverse masses: as FP32 pairs where every mass and its low part are
+// normal FP32 numbers (masses within 1e-27 .. 1e30), else in FP64
+int upload_fp64_mass(axg_handle *h, const std::vector<double> &m, float2 **pair, double **dp) {
+  for (double x : m)
+    if (x != 0.0 && !(std::fabs(x) >= 1e-27 && std::fabs(x) <= 1e30)) return upload(h, dp, m);
+  std::vector<float2> p(m.size());
+  for (size_t k = 0; k < m.size(); ++k) split(m[k], p[k].x, p[k].y);
+  return upload(h, pair, p);
+}
+
 // share: an existing handle on the same mesh (axg_create_sharing) whose
 // plans and mesh-level device buffers are used instead of building new ones
 int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share = nullptr) {
@@ -1708,6 +1721,8 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
     h->inv_mass_f = share->inv_mass_f;
     h->inv_mass_s_dp = share->inv_mass_s_dp;
     h->inv_mass_f_dp = share->inv_mass_f_dp;
+    h->inv_mass_s_pair = share->inv_mass_s_pair;
+    h->inv_mass_f_pair = share->inv_mass_f_pair;
     h->gamma_s = share->gamma_s;
     h->gamma_f = share->gamma_f;
     h->to_fluid = share->to_fluid;
@@ -1722,9 +1737,11 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
     if (!rc && h->absorbing) rc = upload(h, &h->gamma_s, per_point(d->solid_absorbing_gamma, h->igloc_s, h->nglob_s));
     if (!rc && h->nel_f > 0) rc = upload(h, &h->inv_mass_f, per_point(d->inv_mass_fluid, h->igloc_f, h->nglob_f));
     if (!rc && d->inv_mass_rho_dp)
-      rc = upload(h, &h->inv_mass_s_dp, per_point(d->inv_mass_rho_dp, h->igloc_s, h->nglob_s));
+      rc = upload_fp64_mass(h, per_point(d->inv_mass_rho_dp, h->igloc_s, h->nglob_s), &h->inv_mass_s_pair,
+                            &h->inv_mass_s_dp);
     if (!rc && h->nel_f > 0 && d->inv_mass_fluid_dp)
-      rc = upload(h, &h->inv_mass_f_dp, per_point(d->inv_mass_fluid_dp, h->igloc_f, h->nglob_f));
+      rc = upload_fp64_mass(h, per_point(d->inv_mass_fluid_dp, h->igloc_f, h->nglob_f), &h->inv_mass_f_pair,
+                            &h->inv_mass_f_dp);
     if (!rc && h->nel_f > 0 && h->absorbing)
       rc = upload(h, &h->gamma_f, per_point(d->fluid_absorbing_gamma, h->igloc_f, h->nglob_f));
     if (!rc) rc = upload_coupling(h, cf, h->to_fluid);

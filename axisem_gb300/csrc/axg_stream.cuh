@@ -1006,6 +1006,7 @@ struct FluidForce {
   __device__ __forceinline__ float accel(const StreamWork &w, int64_t g) const {
     float sum[1] = {(s0 & kStCoupled) ? w.ffl[g] : 0.f};
     cp.sum(w.df, sum);
+    if (KAHAN && w.fluid.inv_mass_pair) return -mul_pair(w.fluid.inv_mass_pair[g], sum[0]);
     if (KAHAN && w.fluid.inv_mass_dp) return (float)(-w.fluid.inv_mass_dp[g] * (double)sum[0]);  // FP64, one rounding
     return -w.fluid.inv_mass[g] * sum[0];
   }
@@ -1064,13 +1065,13 @@ template <int POLE, int MODE, bool KAHAN>
 struct SolidPoint {
   static constexpr int NC = POLE == POLE_MONO ? 2 : 3;
   static __device__ __forceinline__ int gc(int c) { return (POLE == POLE_MONO && c == 1) ? 2 : c; }
-  float dsp[NC], vel[NC], acc[NC], kc[KAHAN ? NC : 1], kv[KAHAN ? NC : 1], im, gam;
-  double imd;
+  float dsp[NC], vel[NC], acc[NC], kc[KAHAN ? NC : 1], kv[KAHAN ? NC : 1], gam;
+  float2 im;  // (y: the low part of an FP64 inverse mass, else 0)
 
   __device__ __forceinline__ void load(const StateArgs &st, int64_t g) {
-    im = st.inv_mass[g];
+    if (KAHAN && st.inv_mass_pair) im = st.inv_mass_pair[g];
+    else im = make_float2(st.inv_mass[g], 0.f);
     gam = st.gamma ? st.gamma[g] : 0.f;
-    imd = KAHAN && st.inv_mass_dp ? st.inv_mass_dp[g] : 0.0;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       vel[c] = st.v[gc(c)][g];
@@ -1114,13 +1115,12 @@ struct SolidPoint {
         if (KAHAN) dsp[c] = drift_comp(dsp[c], vel[c], st, kc[q]);
         else dsp[c] = dsp[c] + mul2(st.dt, st.dt_lo, vel[c]);
       }
+      // (a symplectic kick doubles the dipole's z component's increment, below)
+      const float f = two && MODE != MODE_SYMPLECTIC ? 2.f * sum[c] : sum[c];
       float a;
-      if (MODE == MODE_SYMPLECTIC)
-        a = KAHAN && st.inv_mass_dp ? (float)(-imd * (double)sum[c]) : -im * sum[c];
-      else if (KAHAN && st.inv_mass_dp)
-        a = (float)(two ? (-2.0 * imd) * (double)sum[c] : -imd * (double)sum[c]);
-      else
-        a = two ? (-2.f * im) * sum[c] : -im * sum[c];
+      if (KAHAN && st.inv_mass_pair) a = -mul_pair(im, f);
+      else if (KAHAN && st.inv_mass_dp) a = (float)(-st.inv_mass_dp[g] * (double)f);  // FP64, one rounding
+      else a = -im.x * f;
       if (st.gamma) a = a - 2.f * gam * vel[c] - gam * gam * dsp[c];
       const float inc = MODE == MODE_SYMPLECTIC
                             ? mul2(two ? 2.f * st.kick : st.kick, two ? 2.f * st.kick_lo : st.kick_lo, a)
