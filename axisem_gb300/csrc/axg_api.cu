@@ -89,9 +89,9 @@ struct DomainDev {
 
 // Order of a domain for the step: element slots, groups, the internal point
 // numbering, and for a patched solid its patches.  A patch's own points (held
-// by it alone, not coupled) are consecutive; the deferred points come after
-// all own points (n_own of them, 0 in a scattered domain, whose points are all
-// left to the point pass).
+// by it alone, not coupled) are consecutive, as are the inner points of a
+// scattered solid's elements (n_own = 9 per element, 0 if a mesh shares any);
+// all other points come after them.
 struct StreamOrder {
   bool patched = false;
   std::vector<int32_t> elem_order;              // slot -> element
@@ -163,7 +163,7 @@ struct axg_handle {
   float *stf = nullptr, *rec = nullptr;
   int32_t *iter = nullptr, *blowup = nullptr, *rec_gidx_d = nullptr;
   int32_t *src_gidx_d = nullptr;
-  std::vector<int32_t> src_patches;  // patches that own source points (at most 8: one per source element)
+  std::vector<int32_t> src_patches;  // patches (scattered: element slots) that own source points, at most 8
   float *src_val_d = nullptr;
   int32_t n_src = 0;
   // gvec I/O in the reference's numbering (made on first use): the solid
@@ -514,6 +514,23 @@ void stream_order(const DomainPlan &pl, const int32_t *igloc, const std::vector<
     }
   }
   std::vector<int32_t> key(nglob, 0);
+  if (split && !patched) {
+    // inner points of one copy, and not coupled (always so on a mesh whose
+    // elements meet in edges and corners)
+    std::vector<uint8_t> copies(nglob, 0), inner(nglob, 0);
+    for (int64_t q = 0; q < 25 * nel; ++q) copies[igloc[q] - 1] = (uint8_t)std::min(2, copies[igloc[q] - 1] + 1);
+    bool all = true;
+    for (int64_t e = 0; e < nel; ++e)
+      for (int q = 0; q < 9; ++q) {
+        const int64_t g = igloc[25 * e + 5 * (q / 3 + 1) + q % 3 + 1] - 1;
+        all = all && copies[g] == 1 && (coupled.empty() || !coupled[g]);
+        inner[g] = 1;
+      }
+    if (all) {
+      o.n_own = 9 * nel;
+      for (int64_t g = 0; g < nglob; ++g) key[g] = !inner[g];
+    }
+  }
   if (patched) {
     for (int64_t g = 0; g < nglob; ++g) {
       key[g] = r1[g] < np || r0[g] == np || (!coupled.empty() && coupled[g]);
@@ -534,6 +551,10 @@ void stream_order(const DomainPlan &pl, const int32_t *igloc, const std::vector<
     return out;
   };
   o.old_of_new = csort(key, 2, csort(r0, np + 1, csort(r1, np + 1, {})));
+  if (!patched && o.n_own > 0)  // the inner points in slot order
+    for (int64_t s = 0; s < nel; ++s)
+      for (int q = 0; q < 9; ++q)
+        o.old_of_new[9 * s + q] = igloc[25 * (int64_t)o.elem_order[s] + 5 * (q / 3 + 1) + q % 3 + 1] - 1;
   o.new_of_old.resize(nglob);
   for (int64_t n = 0; n < nglob; ++n) o.new_of_old[o.old_of_new[n]] = (int32_t)n;
   if (!patched) return;
@@ -679,7 +700,8 @@ int build_domain(axg_handle *h, const axg_mesh_desc *d, bool fluid, bool mesh_pa
     if (o.patched) {
       for (int32_t g : o.def) fill[g - p0 + 1]++;
     } else {
-      for (int64_t q = 0; q < 25 * nel; ++q) fill[ig[q]]++;
+      for (int64_t q = 0; q < 25 * nel; ++q)
+        if (ig[q] > p0) fill[ig[q] - p0]++;
     }
     if (!fluid)
       for (int32_t g : coupled) fill[g - p0 + 1]++;
@@ -693,8 +715,10 @@ int build_domain(axg_handle *h, const axg_mesh_desc *d, bool fluid, bool mesh_pa
       for (size_t q = 0; q < o.def.size(); ++q) ent[fill[o.def[q] - p0]++] = (int32_t)(4 * q);
     } else {
       for (int64_t s = 0; s < nel; ++s)
-        for (int k = 0; k < 25; ++k)
-          ent[fill[ig[25 * (int64_t)o.elem_order[s] + k] - 1]++] = (int32_t)((5 * s + k / 5) * fs + k % 5);
+        for (int k = 0; k < 25; ++k) {
+          const int64_t g = ig[25 * (int64_t)o.elem_order[s] + k] - 1;
+          if (g >= p0) ent[fill[g - p0]++] = (int32_t)((5 * s + k / 5) * fs + k % 5);
+        }
     }
     std::vector<uint8_t> onaxis(nglob, 0);
     for (int64_t e = 0; e < nel; ++e)
@@ -1030,6 +1054,7 @@ void stream_launches(const axg_handle *h, int mode, const StreamWork &base, Fn f
     fn(kPointPass, w);
     w.nb_fp = 0;
   }
+  if (!h->os.patched) w.nb_si = ceil_div(h->os.n_own, kGrpThreads);
   w.nb_sp = ceil_div(h->nglob_s - h->os.n_own, kGrpThreads);
   if (mode == MODE_NEWMARK) w.nb_rec = 1;
   if (stream_blocks(w) > 0) fn(kPointPass, w);
@@ -1691,6 +1716,11 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
   h->n_src = (int32_t)src_g.size();
   for (int32_t g : src_g) {
     if (g >= h->os.n_own) continue;
+    if (!h->os.patched) {
+      if (std::find(h->src_patches.begin(), h->src_patches.end(), g / 9) == h->src_patches.end())
+        h->src_patches.push_back(g / 9);
+      continue;
+    }
     const auto it = std::upper_bound(h->os.patches.begin(), h->os.patches.end(), g,
                                      [](int32_t x, const PatchInfo &p) { return x < p.int_start; });
     // (a patch without own points starts where the next does)

@@ -141,7 +141,7 @@ struct StreamDomain {
   const PatchInfo *patches;
   const GroupMeta *groups;
   const int32_t *def;       // the deferred points' global indices, patch by patch
-  int32_t src_patch[8];     // patches whose own points carry source terms
+  int32_t src_patch[8];     // patches whose own points (scattered: element slots whose inner points) carry source terms
   int32_t n_src_patch, n_patches;
   int64_t n_off;            // scattered solid: elements off the axis
   int64_t nel, nglob, n_m0, n_ent, n_fel, n_def;
@@ -149,8 +149,9 @@ struct StreamDomain {
 
 // One launch of a solve's step.  Its CTAs are, in order: element-pass CTAs of
 // the solid (one per patch, or kGrpWarps groups each), of the fluid groups,
-// the rows of the coupling into the fluid; or point-pass CTAs of the solid
-// points [p0, nglob), of the fluid points, and the receivers' CTA.
+// the rows of the coupling into the fluid; or point-pass CTAs of a scattered
+// solid's inner points [0, p0), of the solid points [p0, nglob), of the fluid
+// points, and the receivers' CTA.
 struct StreamWork {
   StreamDomain ds, df;
   StateArgs solid, fluid;
@@ -159,7 +160,7 @@ struct StreamWork {
   const uint8_t *axmask;    // the solid's per-point axis mask bits or null
   CgArgs cg;
   int32_t p0;               // first solid point of the point pass
-  int32_t nb_se, nb_fe, nb_cp, nb_sp, nb_fp, nb_rec;  // CTAs per role
+  int32_t nb_se, nb_fe, nb_cp, nb_si, nb_sp, nb_fp, nb_rec;  // CTAs per role
   int32_t prefetch;         // element pass: CTAs ahead whose blocks are prefetched into L2 (0: none)
   int32_t *iter_p;          // the step number of the point pass
   const int32_t *memvar_gidx;  // memvar_kernel: each element slot's 25 points
@@ -1156,6 +1157,39 @@ struct SolidPoint {
   }
 };
 
+// An inner GLL point of an element of a scattered solid (nine per element, 9/16
+// of the points): one copy, whose place follows from the point's number
+// 9 slot + 3 (j - 1) + i - 1, so no index is read: steps of 353 000 points took
+// 25.1 us with all points through the lists below and take 24.8 (compensated),
+// 15.4 / 13.9 without; with cg4 on 2.2 million points 49.5 / 47.6.  (Finished by
+// the element pass itself they cost more: its chain is the longer one.)
+template <int POLE, int MODE, bool KAHAN>
+__device__ __forceinline__ void inner_point(const StreamWork &w, int32_t g) {
+  using S = SolidPoint<POLE, MODE, KAHAN>;
+  constexpr int NC = S::NC;
+  const StreamDomain &d = w.ds;
+  const StateArgs &st = w.solid;
+  const int32_t slot = g / 9, q = g - 9 * slot;
+  const int64_t e = ((int64_t)slot * 5 + q / 3 + 1) * solid_fs(POLE) + q % 3 + 1;
+  pdl_wait();
+  const bool stopped = MODE != MODE_FORCE && *st.blowup != 0;
+  S pt;
+  if (MODE != MODE_FORCE) pt.load(st, g);
+  if (!AXG_BOUND(e + 5 * (NC - 1), d.n_fel, 70)) return;
+  float sum[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) sum[c] = 0.f + d.fel[e + 5 * c];
+  if (MODE == MODE_FORCE) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) st.f[S::gc(c)][g] = sum[c];
+    return;
+  }
+  if (stopped) return;
+  for (int k = 0; k < d.n_src_patch; ++k)
+    if (d.src_patch[k] == slot) S::source(st, *w.iter_p, g, sum);
+  pt.finish(st, g, false, sum);
+}
+
 // A solid point of the point pass: the coupling, then the copies' (the
 // patches') sums in order.
 template <int POLE, int MODE, bool PATCH, bool KAHAN>
@@ -1164,7 +1198,7 @@ __device__ __forceinline__ void solid_point(const StreamWork &w, int64_t g) {
   constexpr int NC = S::NC;
   const StreamDomain &d = w.ds;
   const StateArgs &st = w.solid;
-  const int64_t r = PATCH ? g - w.p0 : g;
+  const int64_t r = g - w.p0;
   const uint32_t s0 = (uint32_t)d.start[r], s1 = (uint32_t)d.start[r + 1] & kStMask;
   const bool coupled = (s0 & kStCoupled) != 0;
   const Copies<NC, PATCH ? 1 : 5> cps(d, (s0 & kStMask) + (coupled ? 1 : 0), s1);
@@ -1454,11 +1488,17 @@ __global__ void __launch_bounds__(kGrpThreads) point_kernel(const __grid_constan
   pdl_trigger();
   int b = blockIdx.x;
   const StreamWork &w = p.find(b);
-  if (MODE == MODE_NEWMARK && b == w.nb_sp + w.nb_fp) {
+  if (MODE == MODE_NEWMARK && b == w.nb_si + w.nb_sp + w.nb_fp) {
     pdl_wait();
     if (w.nb_rec > 0) stream_receivers<POLE>(w);
     return;
   }
+  if (!PATCH && b < w.nb_si) {
+    const int32_t g = b * kGrpThreads + threadIdx.x;
+    if (g < w.p0) inner_point<POLE, MODE, KAHAN>(w, g);
+    return;
+  }
+  b -= w.nb_si;
   if (b < w.nb_sp) {
     const int64_t g = (int64_t)w.p0 + (int64_t)b * kGrpThreads + threadIdx.x;
     if (g < w.ds.nglob) solid_point<POLE, MODE, PATCH, KAHAN>(w, g);

@@ -18,7 +18,7 @@ struct StreamKernel {
 
 // CTAs of a launch's work
 inline int32_t stream_blocks(const StreamWork &w) {
-  return w.nb_se + w.nb_fe + w.nb_cp + w.nb_sp + w.nb_fp + w.nb_rec;
+  return w.nb_se + w.nb_fe + w.nb_cp + w.nb_si + w.nb_sp + w.nb_fp + w.nb_rec;
 }
 
 // One launch for a solve or for several solves (with programmatic stream

@@ -34,6 +34,26 @@ def test_group_remainders(gpu_lib, orc, pole, ni, nj, axial):
     assert rel(f, orc.stiffness_assembled(m, u, np.float64)) <= 1e-5
 
 
+@pytest.mark.parametrize("pole", [0, 1, 2])
+def test_inner_points_of_two_elements(gpu_lib, orc, pole):
+    """Inner points are summed by their place in the contributions unless a mesh
+    shares one between elements: the general path for all of its points.  (The
+    oracle sums edge points only; the two elements' inner forces are added here.)"""
+    m = structured_mesh(7, 5, pole, axial="column", seed=6)
+    u = random_gvec(m, seed=7)
+    ig = m.igloc_solid.copy()
+    a, b = ig[25 * 23 + 12] - 1, ig[25 * 9 + 12] - 1
+    u[b] = u[a]
+    want = orc.stiffness_assembled(m, u, np.float64)
+    want[a] += want[b]
+    want[b] = 0.0
+    ig[25 * 9 + 12] = a + 1
+    m.igloc_solid = ig
+    with Solver(m) as s:
+        f = s.stiffness_assembled(u)
+    assert rel(f, want) <= 1e-5
+
+
 PATCHED = (367, 359)   # 131 753 elements: patched; not multiples of a patch's 8 x 8
 
 
