@@ -941,14 +941,20 @@ cudaError_t stream_ctas(int pole, const StreamKernel &k, int *per_sm) {
   return stream_elem_ctas<POLE_QUAD>(k, per_sm);
 }
 
+// A mesh whose element blocks do not fit L2 streams them from HBM once per
+// step; a smaller one finds them there.
+constexpr int64_t kL2Resident = 64 << 20;
+bool streamed(const axg_handle *h) { return h->nel_s * 100 * (n_terms(h->pole) + 1) > kL2Resident; }
+
 // the kernel of a launch of the handle's step
 StreamKernel step_kernel(const axg_handle *h, int kind) {
-  return {kind, h->scheme == AXG_SCHEME_NEWMARK2 ? MODE_NEWMARK : MODE_SYMPLECTIC, h->os.patched, h->anel, h->kahan};
+  return {kind,    h->scheme == AXG_SCHEME_NEWMARK2 ? MODE_NEWMARK : MODE_SYMPLECTIC, h->os.patched, h->anel, h->kahan,
+          streamed(h)};
 }
 
 // resident CTAs per SM of the element passes the handle's modes select
 int prepare_kernels(axg_handle *h) {
-  CK(stream_ctas(h->pole, {kElemPass, MODE_FORCE, h->os.patched, false, false}, &h->elem_ctas_force));
+  CK(stream_ctas(h->pole, {kElemPass, MODE_FORCE, h->os.patched, false, false, false}, &h->elem_ctas_force));
   CK(stream_ctas(h->pole, step_kernel(h, kElemPass), &h->elem_ctas_step));
   return AXG_OK;
 }
@@ -994,10 +1000,6 @@ StreamDomain stream_domain(const DomainDev &dd, int64_t nel, int64_t nglob) {
   return a;
 }
 
-// A mesh whose element blocks do not fit L2 streams them from HBM once per
-// step; a smaller one finds them there.
-constexpr int64_t kL2Resident = 64 << 20;
-
 // the arguments all launches of a step (a stage) share
 StreamWork stream_work(axg_handle *h, int mode, const StateArgs &ss, const StateArgs &fs) {
   StreamWork w{};
@@ -1012,8 +1014,7 @@ StreamWork stream_work(axg_handle *h, int mode, const StateArgs &ss, const State
   w.cg = h->cg;
   w.iter_p = h->iter_p;
   w.p0 = (int32_t)h->os.n_own;
-  const int64_t bytes = h->nel_s * 100 * (n_terms(h->pole) + 1);
-  if (bytes > kL2Resident) w.prefetch = (mode == MODE_FORCE ? h->elem_ctas_force : h->elem_ctas_step) * h->num_sms;
+  if (streamed(h)) w.prefetch = (mode == MODE_FORCE ? h->elem_ctas_force : h->elem_ctas_step) * h->num_sms;
   if (mode == MODE_FORCE) return w;
   w.rec = rec_work(h, ss);
   if (h->nel_f > 0) {
@@ -1086,7 +1087,7 @@ void launch_anel_full(axg_handle *h, cudaStream_t s, bool update) {
 void enqueue_force(axg_handle *h, cudaStream_t s) {
   const StreamWork w = stream_work(h, MODE_FORCE, solid_state(h), StateArgs{});
   stream_launches(h, MODE_FORCE, w, [&](int kind, const StreamWork &x) {
-    launch_stream(h, {kind, MODE_FORCE, h->os.patched, false, false}, x, s);
+    launch_stream(h, {kind, MODE_FORCE, h->os.patched, false, false, false}, x, s);
   });
 }
 

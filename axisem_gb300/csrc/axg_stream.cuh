@@ -1463,19 +1463,23 @@ __device__ __forceinline__ void elem_cta(const P &p, const SpecDev &sp, float *x
   if (q < w.to_fluid.n) couple_row<POLE, MODE, KAHAN>(w, q);
 }
 
-// the element pass of meshes whose contributions stay in L2 (up to 128
-// registers, four CTAs per SM; with attenuation the memory variables need
-// more, three)
-template <int POLE, int MODE, bool ANEL, bool KAHAN, class P>
-__global__ void __launch_bounds__(kGrpThreads, ANEL ? 3 : 4)
+// The element pass of meshes whose contributions stay in L2.  CTAs: per SM; 4
+// (up to 128 registers) where the blocks come from L2, 3 (up to 168) where a
+// dipole's or quadrupole's come from HBM: more of a column's rows in flight per
+// warp then weigh more than warps.  With attenuation the memory variables need
+// the registers: 3.
+template <int POLE, int MODE, bool ANEL, bool KAHAN, int CTAS, class P>
+__global__ void __launch_bounds__(kGrpThreads, CTAS)
     scatter_kernel(const __grid_constant__ P p, const __grid_constant__ SpecDev sp) {
   __shared__ __align__(16) float xch[kGrpWarps * kXchFloats];
   __shared__ float scr[ANEL ? kGrpWarps * kScFloats : 1];
   elem_cta<POLE, false, MODE, ANEL, KAHAN>(p, sp, xch, scr, nullptr);
 }
-// the element pass of larger meshes
+// The element pass of larger meshes: 3 CTAs per SM took 21.6 ms where 4 took
+// 23.1 (30 steps, quadrupole, 1 048 576 elements); a monopole keeps 4 (18.1 ms
+// against 20.3).
 template <int POLE, int MODE, bool ANEL, bool KAHAN, class P>
-__global__ void __launch_bounds__(kGrpThreads, ANEL ? 3 : 4)
+__global__ void __launch_bounds__(kGrpThreads, ANEL || POLE != POLE_MONO ? 3 : 4)
     patch_kernel(const __grid_constant__ P p, const __grid_constant__ SpecDev sp) {
   __shared__ __align__(16) float xch[kGrpWarps * kXchFloats];
   __shared__ float scr[ANEL ? kGrpWarps * kScFloats : 1];

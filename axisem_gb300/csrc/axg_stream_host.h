@@ -10,10 +10,11 @@ namespace axg {
 
 enum StreamKind { kElemPass = 0, kPointPass = 1 };
 
-// what a launch of a step is: its kernel
+// what a launch of a step is: its kernel (streamed: the element blocks come
+// from HBM)
 struct StreamKernel {
   int kind, mode;
-  bool patched, anel, kahan;
+  bool patched, anel, kahan, streamed;
 };
 
 // CTAs of a launch's work

@@ -22,9 +22,21 @@ cudaError_t launch(void (*kernel)(KArgs...), unsigned grid, cudaStream_t s, bool
 unsigned blocks(const StreamOne &p) { return (unsigned)stream_blocks(p.w); }
 unsigned blocks(const StreamMany &p) { return (unsigned)p.start[p.n]; }
 
+// CTAs per SM of the scattered element pass.  Quadrupole steps, 4 / 3 CTAs: from
+// L2 12.9 / 14.0 us on 13 390 elements, from HBM 20.1 / 17.0 on 18 944, 23.9 /
+// 23.6 on 25 802, 32.4 / 33.2 on 32 298 (3 waves either way), 73.2 / 71.3 on
+// 70 528.  Several solves' launches, whose waves fill, keep 4: six solves on
+// 5 664 elements each 9.67 / 9.95 ms for 100 steps.
 template <int POLE, int MODE, bool ANEL, bool KAHAN, class P>
-auto patched_or(bool patched) -> void (*)(P, SpecDev) {
-  return patched ? patch_kernel<POLE, MODE, ANEL, KAHAN, P> : scatter_kernel<POLE, MODE, ANEL, KAHAN, P>;
+auto scatter_of(const StreamKernel &k) -> void (*)(P, SpecDev) {
+  if constexpr (ANEL) return scatter_kernel<POLE, MODE, ANEL, KAHAN, 3, P>;
+  else if constexpr (POLE == POLE_MONO || P::kMany) return scatter_kernel<POLE, MODE, ANEL, KAHAN, 4, P>;
+  else return k.streamed ? scatter_kernel<POLE, MODE, ANEL, KAHAN, 3, P> : scatter_kernel<POLE, MODE, ANEL, KAHAN, 4, P>;
+}
+
+template <int POLE, int MODE, bool ANEL, bool KAHAN, class P>
+auto patched_or(const StreamKernel &k) -> void (*)(P, SpecDev) {
+  return k.patched ? patch_kernel<POLE, MODE, ANEL, KAHAN, P> : scatter_of<POLE, MODE, ANEL, KAHAN, P>(k);
 }
 
 // The scattered element pass of a Newmark step does not depend on the
@@ -32,20 +44,20 @@ auto patched_or(bool patched) -> void (*)(P, SpecDev) {
 // finishes points.
 template <int POLE, class P>
 auto elem_kernel(const StreamKernel &k) -> void (*)(P, SpecDev) {
-  if (k.mode == MODE_FORCE) return patched_or<POLE, MODE_FORCE, false, false, P>(k.patched);
+  if (k.mode == MODE_FORCE) return patched_or<POLE, MODE_FORCE, false, false, P>(k);
   if (k.mode == MODE_NEWMARK) {
     if (!k.patched)
-      return k.anel ? scatter_kernel<POLE, MODE_NEWMARK, true, false, P>
-                    : scatter_kernel<POLE, MODE_NEWMARK, false, false, P>;
+      return k.anel ? scatter_of<POLE, MODE_NEWMARK, true, false, P>(k)
+                    : scatter_of<POLE, MODE_NEWMARK, false, false, P>(k);
     if (k.anel)
       return k.kahan ? patch_kernel<POLE, MODE_NEWMARK, true, true, P> : patch_kernel<POLE, MODE_NEWMARK, true, false, P>;
     return k.kahan ? patch_kernel<POLE, MODE_NEWMARK, false, true, P> : patch_kernel<POLE, MODE_NEWMARK, false, false, P>;
   }
   if (k.anel)
-    return k.kahan ? patched_or<POLE, MODE_SYMPLECTIC, true, true, P>(k.patched)
-                   : patched_or<POLE, MODE_SYMPLECTIC, true, false, P>(k.patched);
-  return k.kahan ? patched_or<POLE, MODE_SYMPLECTIC, false, true, P>(k.patched)
-                 : patched_or<POLE, MODE_SYMPLECTIC, false, false, P>(k.patched);
+    return k.kahan ? patched_or<POLE, MODE_SYMPLECTIC, true, true, P>(k)
+                   : patched_or<POLE, MODE_SYMPLECTIC, true, false, P>(k);
+  return k.kahan ? patched_or<POLE, MODE_SYMPLECTIC, false, true, P>(k)
+                 : patched_or<POLE, MODE_SYMPLECTIC, false, false, P>(k);
 }
 
 template <int POLE, int MODE, class P>

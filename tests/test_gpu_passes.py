@@ -67,6 +67,30 @@ def test_patched_stiffness(gpu_lib, orc, pole):
     assert rel(f, orc.stiffness_assembled(m, u, np.float64)) <= 1e-5
 
 
+@pytest.mark.parametrize("pole,comp", [(0, False), (1, False), (1, True), (2, False)])
+def test_scattered_steps_from_hbm(gpu_lib, orc, pole, comp):
+    """Scattered solids whose element blocks exceed what L2 keeps, with a group
+    of fewer elements at the end."""
+    n = 4
+    m = coupled_mesh(187, 151, 5, pole, niter=n, num_rec=5, seis_it=1, terms="pole", src_row=7)
+    u = random_gvec(m, seed=8)
+    if pole == 0:
+        u[:, 1] = 0.0
+    t = orc.TimeLoop(m, np.float64)
+    t.disp[...] = gvec_to_elemental(m, u)
+    assert t.run(1, n) == 0
+    comps = [0, 2] if pole == 0 else [0, 1, 2]
+    with Solver(m) as s:
+        s.set_compensated(comp)
+        f = s.stiffness_assembled(u)
+        assert rel(f, orc.stiffness_assembled(m, u, np.float64)) <= 1e-5
+        s.upload_disp(u)
+        s.run(1, n)
+        assert rel(s.get_state(_abi.FIELD_DISP)[..., comps], t.disp[..., comps]) <= 1e-4
+        assert rel(s.get_state(_abi.FIELD_VELO)[..., comps], t.velo[..., comps]) <= 1e-4
+        assert rel(s.get_state(_abi.FIELD_CHI), t.chi) <= 1e-4
+
+
 @pytest.mark.parametrize("pole,mode,absorbing", [(0, "plain", True), (1, "plain", False), (2, "comp", False),
                                                  (1, "comp", True), (2, "symplec4", False)])
 def test_patched_steps(gpu_lib, orc, pole, mode, absorbing):
