@@ -941,9 +941,13 @@ cudaError_t stream_ctas(int pole, const StreamKernel &k, int *per_sm) {
   return stream_elem_ctas<POLE_QUAD>(k, per_sm);
 }
 
-// A mesh whose element blocks do not fit L2 streams them from HBM once per
-// step; a smaller one finds them there.
-constexpr int64_t kL2Resident = 64 << 20;
+// A mesh whose element blocks do not stay in L2 (beside the state and the
+// contributions, about as much again) streams them from HBM once per step, with
+// prefetches and evict-first reads; a smaller one finds them there.  Steps
+// without / with these, sphere meshes: 30 MB of blocks 12.3 / 13.1 us
+// (monopole), 36 MB 12.9 / 13.9 (quadrupole), 41 MB 16.9 / 15.8 (monopole),
+// 47 MB 17.5 / 16.4 (dipole), 51 MB 18.6 / 17.1, 64 MB 26.5 / 22.4 (dipole).
+constexpr int64_t kL2Resident = 38 << 20;
 bool streamed(const axg_handle *h) { return h->nel_s * 100 * (n_terms(h->pole) + 1) > kL2Resident; }
 
 // the kernel of a launch of the handle's step
