@@ -1140,9 +1140,9 @@ void launch_anel_memvar(axg_handle *h, cudaStream_t s) {
   StreamOne p{stream_work(h, MODE_SYMPLECTIC, solid_state(h), fluid_state(h))};
   p.w.memvar_gidx = h->slot_gidx;
   const int32_t n = (int32_t)h->os.groups.size();
-  if (h->pole == AXG_MONOPOLE) stream_memvar<POLE_MONO>(h->os.patched, p, h->spec, n, s);
-  else if (h->pole == AXG_DIPOLE) stream_memvar<POLE_DI>(h->os.patched, p, h->spec, n, s);
-  else stream_memvar<POLE_QUAD>(h->os.patched, p, h->spec, n, s);
+  if (h->pole == AXG_MONOPOLE) stream_memvar<POLE_MONO>(p, h->spec, n, s);
+  else if (h->pole == AXG_DIPOLE) stream_memvar<POLE_DI>(p, h->spec, n, s);
+  else stream_memvar<POLE_QUAD>(p, h->spec, n, s);
 }
 
 // One step of symplectic_time_loop (SOLVER/time_evol_wave.F90:587-727):

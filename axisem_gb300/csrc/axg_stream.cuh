@@ -1271,8 +1271,8 @@ struct PatchSmem {
 // elements share points accumulate in the order of their rounds (a group
 // waits until the groups of earlier rounds have accumulated; its stiffness,
 // most of the work, comes before the wait), those of one round share none.
-template <int POLE, int MODE, bool ANEL, bool KAHAN>
-__device__ __forceinline__ void patch_cta(const StreamWork &w, const SpecDev &sp, int32_t p, float *xw, float *sc,
+template <int POLE, int MODE, bool KAHAN>
+__device__ __forceinline__ void patch_cta(const StreamWork &w, const SpecDev &sp, int32_t p, float *xw,
                                           PatchSmem<POLE> &s) {
   using S = SolidPoint<POLE, MODE, KAHAN>;
   constexpr int NC = S::NC;
@@ -1315,18 +1315,11 @@ __device__ __forceinline__ void patch_cta(const StreamWork &w, const SpecDev &sp
         const PatchInfo pn = d.patches[p + w.prefetch];
         if (warp < pn.n_groups) h = d.groups[pn.group0 + warp];
       }
-      if (h.n > 0 && lane == 0) {
-        prefetch_l2(d.blocks + (int64_t)h.slot0 * row, h.n * row * 4);
-        if (ANEL) {
-          prefetch_l2(w.cg.consts + (int64_t)h.slot0 * 48, h.n * 48 * 4);
-          prefetch_l2(w.cg.state + (int64_t)h.slot0 * 4 * cg_state_floats(w.cg.nsls),
-                      h.n * 16 * cg_state_floats(w.cg.nsls));
-        }
-      }
+      if (h.n > 0 && lane == 0) prefetch_l2(d.blocks + (int64_t)h.slot0 * row, h.n * row * 4);
     }
     bool turn = false;
-    solid_group<POLE, true, MODE, ANEL, KAHAN>(
-        w, sp, g, xw, sc, pi.int_start, pi.n_int, s.def,
+    solid_group<POLE, true, MODE, false, KAHAN>(
+        w, sp, g, xw, nullptr, pi.int_start, pi.n_int, s.def,
         [&]() {
           if (!waited) {
             pdl_wait();
@@ -1445,7 +1438,7 @@ __device__ __forceinline__ void elem_cta(const P &p, const SpecDev &sp, float *x
       *w.iter_p = *w.solid.iter;
     }
     if constexpr (PATCH) {
-      patch_cta<POLE, MODE, ANEL, KAHAN>(w, sp, b, xw, sc, *ps);
+      patch_cta<POLE, MODE, KAHAN>(w, sp, b, xw, *ps);
     } else {
       const int32_t grp = b * kGrpWarps + warp;
       if (grp < scatter_groups(w.ds.n_off, w.ds.nel)) scatter_group<POLE, MODE, ANEL, KAHAN>(w, sp, grp, xw, sc);
@@ -1475,16 +1468,15 @@ __global__ void __launch_bounds__(kGrpThreads, CTAS)
   __shared__ float scr[ANEL ? kGrpWarps * kScFloats : 1];
   elem_cta<POLE, false, MODE, ANEL, KAHAN>(p, sp, xch, scr, nullptr);
 }
-// The element pass of larger meshes: 3 CTAs per SM took 21.6 ms where 4 took
+// The element pass of larger meshes (without coarse-grained attenuation): 3 CTAs per SM took 21.6 ms where 4 took
 // 23.1 (30 steps, quadrupole, 1 048 576 elements); a monopole keeps 4 (18.1 ms
 // against 20.3).
-template <int POLE, int MODE, bool ANEL, bool KAHAN, class P>
-__global__ void __launch_bounds__(kGrpThreads, ANEL || POLE != POLE_MONO ? 3 : 4)
+template <int POLE, int MODE, bool KAHAN, class P>
+__global__ void __launch_bounds__(kGrpThreads, POLE != POLE_MONO ? 3 : 4)
     patch_kernel(const __grid_constant__ P p, const __grid_constant__ SpecDev sp) {
   __shared__ __align__(16) float xch[kGrpWarps * kXchFloats];
-  __shared__ float scr[ANEL ? kGrpWarps * kScFloats : 1];
   __shared__ PatchSmem<POLE> ps;
-  elem_cta<POLE, true, MODE, ANEL, KAHAN>(p, sp, xch, scr, &ps);
+  elem_cta<POLE, true, MODE, false, KAHAN>(p, sp, xch, nullptr, &ps);
 }
 
 template <int POLE, int MODE, bool PATCH, bool KAHAN, class P>
@@ -1515,11 +1507,11 @@ __global__ void __launch_bounds__(kGrpThreads) point_kernel(const __grid_constan
 // time_step_memvars (SOLVER/attenuation.f90:81-202) once per step of the
 // symplectic loop, from the drifted displacement: the element pass's first
 // stage and memory-variable update alone, a warp per group.
-template <int POLE, bool PATCH>
+template <int POLE>
 __global__ void __launch_bounds__(kGrpThreads, 4)
     memvar_kernel(const __grid_constant__ StreamOne p, const __grid_constant__ SpecDev sp, int32_t n_groups) {
   __shared__ __align__(16) float xch[kGrpWarps * kXchFloats];
-  using G = SolidGrp<POLE, PATCH>;
+  using G = SolidGrp<POLE, false>;
   constexpr int NC = G::NC;
   const StreamWork &w = p.w;
   if (*w.solid.blowup) return;
@@ -1528,7 +1520,7 @@ __global__ void __launch_bounds__(kGrpThreads, 4)
   if (grp >= n_groups) return;
   const int32_t *ids = w.memvar_gidx;
   float *xw = xch + warp * kXchFloats;
-  const GroupMeta g = PATCH ? w.ds.groups[grp] : scatter_meta(grp, w.ds.n_off, w.ds.nel);
+  const GroupMeta g = scatter_meta(grp, w.ds.n_off, w.ds.nel);
   const int nl = 5 * g.n;
   const int ll = lane < nl ? lane : nl - 1;
   const int e = ll / 5, j = ll % 5, e5 = ll - j;

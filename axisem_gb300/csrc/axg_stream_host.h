@@ -30,7 +30,7 @@ cudaError_t stream_launch(const StreamKernel &k, const StreamOne &p, const SpecD
 template <int POLE>
 cudaError_t stream_launch(const StreamKernel &k, const StreamMany &p, const SpecDev &sp, cudaStream_t s);
 template <int POLE>
-cudaError_t stream_memvar(bool patched, const StreamOne &p, const SpecDev &sp, int32_t n_groups, cudaStream_t s);
+cudaError_t stream_memvar(const StreamOne &p, const SpecDev &sp, int32_t n_groups, cudaStream_t s);
 template <int POLE>
 cudaError_t stream_elem_ctas(const StreamKernel &k, int *per_sm);
 #ifdef AXG_DEVICE_CHECKS

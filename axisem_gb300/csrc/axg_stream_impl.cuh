@@ -34,9 +34,9 @@ auto scatter_of(const StreamKernel &k) -> void (*)(P, SpecDev) {
   else return k.streamed ? scatter_kernel<POLE, MODE, ANEL, KAHAN, 3, P> : scatter_kernel<POLE, MODE, ANEL, KAHAN, 4, P>;
 }
 
-template <int POLE, int MODE, bool ANEL, bool KAHAN, class P>
+template <int POLE, int MODE, bool KAHAN, class P>
 auto patched_or(const StreamKernel &k) -> void (*)(P, SpecDev) {
-  return k.patched ? patch_kernel<POLE, MODE, ANEL, KAHAN, P> : scatter_of<POLE, MODE, ANEL, KAHAN, P>(k);
+  return k.patched ? patch_kernel<POLE, MODE, KAHAN, P> : scatter_of<POLE, MODE, false, KAHAN, P>(k);
 }
 
 // The scattered element pass of a Newmark step does not depend on the
@@ -44,20 +44,17 @@ auto patched_or(const StreamKernel &k) -> void (*)(P, SpecDev) {
 // finishes points.
 template <int POLE, class P>
 auto elem_kernel(const StreamKernel &k) -> void (*)(P, SpecDev) {
-  if (k.mode == MODE_FORCE) return patched_or<POLE, MODE_FORCE, false, false, P>(k);
+  if (k.mode == MODE_FORCE) return patched_or<POLE, MODE_FORCE, false, P>(k);
   if (k.mode == MODE_NEWMARK) {
     if (!k.patched)
       return k.anel ? scatter_of<POLE, MODE_NEWMARK, true, false, P>(k)
                     : scatter_of<POLE, MODE_NEWMARK, false, false, P>(k);
-    if (k.anel)
-      return k.kahan ? patch_kernel<POLE, MODE_NEWMARK, true, true, P> : patch_kernel<POLE, MODE_NEWMARK, true, false, P>;
-    return k.kahan ? patch_kernel<POLE, MODE_NEWMARK, false, true, P> : patch_kernel<POLE, MODE_NEWMARK, false, false, P>;
+    return k.kahan ? patch_kernel<POLE, MODE_NEWMARK, true, P> : patch_kernel<POLE, MODE_NEWMARK, false, P>;
   }
   if (k.anel)
-    return k.kahan ? patched_or<POLE, MODE_SYMPLECTIC, true, true, P>(k)
-                   : patched_or<POLE, MODE_SYMPLECTIC, true, false, P>(k);
-  return k.kahan ? patched_or<POLE, MODE_SYMPLECTIC, false, true, P>(k)
-                 : patched_or<POLE, MODE_SYMPLECTIC, false, false, P>(k);
+    return k.kahan ? scatter_of<POLE, MODE_SYMPLECTIC, true, true, P>(k)
+                   : scatter_of<POLE, MODE_SYMPLECTIC, true, false, P>(k);
+  return k.kahan ? patched_or<POLE, MODE_SYMPLECTIC, true, P>(k) : patched_or<POLE, MODE_SYMPLECTIC, false, P>(k);
 }
 
 template <int POLE, int MODE, class P>
@@ -88,9 +85,8 @@ cudaError_t stream_launch(const StreamKernel &k, const StreamMany &p, const Spec
 }
 
 template <int POLE>
-cudaError_t stream_memvar(bool patched, const StreamOne &p, const SpecDev &sp, int32_t n_groups, cudaStream_t s) {
-  return launch(patched ? memvar_kernel<POLE, true> : memvar_kernel<POLE, false>,
-                (unsigned)((n_groups + kGrpWarps - 1) / kGrpWarps), s, false, p, sp, n_groups);
+cudaError_t stream_memvar(const StreamOne &p, const SpecDev &sp, int32_t n_groups, cudaStream_t s) {
+  return launch(memvar_kernel<POLE>, (unsigned)((n_groups + kGrpWarps - 1) / kGrpWarps), s, false, p, sp, n_groups);
 }
 
 template <int POLE>
@@ -110,7 +106,7 @@ template cudaError_t stream_launch<AXG_STREAM_POLE>(const StreamKernel &, const 
                                                     cudaStream_t);
 template cudaError_t stream_launch<AXG_STREAM_POLE>(const StreamKernel &, const StreamMany &, const SpecDev &,
                                                     cudaStream_t);
-template cudaError_t stream_memvar<AXG_STREAM_POLE>(bool, const StreamOne &, const SpecDev &, int32_t, cudaStream_t);
+template cudaError_t stream_memvar<AXG_STREAM_POLE>(const StreamOne &, const SpecDev &, int32_t, cudaStream_t);
 template cudaError_t stream_elem_ctas<AXG_STREAM_POLE>(const StreamKernel &, int *);
 
 }  // namespace axg
