@@ -246,9 +246,9 @@ __device__ __forceinline__ float drift_comp(float d, float v, const StateArgs &s
 // (float)(m x) for an FP64 factor m held as an FP32 pair m.x + m.y: the product
 // of the high part and its exact rounding error, with the low part's product.
 // Equal to the FP64 product rounded once but for values within about 2^-20
-// of an ulp from a tie.  FP64 runs at 1/64 of the FP32 rate here: on 353 000
-// points of three components a compensated step took 25.6 us with FP64
-// products and takes 23.2 with pairs; errors against FP64 are alike (2.5e-7).
+// of an ulp from a tie.  FP64 runs at 1/64 of the FP32 rate here: on 305 000
+// points of three components a compensated step took 27.6 us with FP64
+// products and took 25.1 with pairs; errors against FP64 are alike (2.5e-7).
 __device__ __forceinline__ float mul_pair(float2 m, float x) {
   const float p = __fmul_rn(m.x, x);
   return __fadd_rn(p, fmaf(m.y, x, fmaf(m.x, x, -p)));

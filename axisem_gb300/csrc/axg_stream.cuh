@@ -292,7 +292,44 @@ __device__ __forceinline__ constexpr bool col_masked(int c) {
 // S2 and the local part before the second stage makes their contraction part
 // of the elastic one.
 constexpr int kCgBatch = 5;  // solids whose memory variables are in flight together
-template <int POLE, bool UPDATE>
+
+// What cg_point reads, copied to shared memory by the cg lane itself while its
+// warp gathers the displacements: the constants before the step's wait, the
+// state of the first kCgBatch solids and the last source terms after it.
+// In a warp's scratch `sc`, after the 9 results per cg lane.  Dipole steps with
+// 5 solids took 133.3 us on 99 450 elements and 371.6 on 278 297 with these
+// read where they are used, and take 131.9 and 369.2.  (Held in registers from
+// the gather on they spill: 157.)
+constexpr int kScConst = 9 * kCgLanes, kScState = kScConst + 12 * kCgLanes,
+              kScTr = kScState + 6 * (kCgBatch + 1) * kCgLanes;
+constexpr int kScFloats = kScTr + kCgLanes;  // per warp
+static_assert(kScConst % 4 == 0 && kScState % 2 == 0 && kScFloats % 4 == 0, "aligned copies");
+__device__ __forceinline__ void cg_stage_consts(const CgArgs &cg, float *sc, const GroupMeta &g, int lane) {
+  const int nl = 4 * g.n;
+  if (lane >= nl) return;
+  const float *cs = cg.consts + (int64_t)g.slot0 * 48 + 4 * lane;
+#pragma unroll
+  for (int r = 0; r < 3; ++r) cp_async16(sc + kScConst + 4 * (r * kCgLanes + lane), cs + (int64_t)4 * r * nl);
+}
+__device__ __forceinline__ void cg_stage_state(const CgArgs &cg, float *sc, const GroupMeta &g, int lane) {
+  const int nl = 4 * g.n, nsls = cg.nsls;
+  if (lane >= nl) return;
+  const float *b = cg.state + (int64_t)g.slot0 * 4 * cg_state_floats(nsls);
+  float *s = sc + kScState + 2 * lane;
+#pragma unroll
+  for (int w = 0; w < 3; ++w)
+    cp_async8(s + 2 * (3 * kCgBatch + w) * kCgLanes, b + 2 * ((int64_t)(3 * nsls + w) * nl + lane));
+  cp_async4(sc + kScTr + lane, b + 6 * (nsls + 1) * nl + lane);
+#pragma unroll
+  for (int q = 0; q < kCgBatch; ++q)
+    if (q < nsls)
+#pragma unroll
+      for (int w = 0; w < 3; ++w)
+        cp_async8(s + 2 * (3 * q + w) * kCgLanes, b + 2 * ((int64_t)(3 * q + w) * nl + lane));
+}
+
+// STAGED: what the two functions above copied is read from there.
+template <int POLE, bool UPDATE, bool STAGED>
 __device__ __forceinline__ void cg_point(const CgArgs &cg, const float *xw, float *sc, const GroupMeta &g, int lane,
                                          bool mine) {
   constexpr int NC = POLE == POLE_MONO ? 2 : 3;
@@ -301,7 +338,11 @@ __device__ __forceinline__ void cg_point(const CgArgs &cg, const float *xw, floa
   const int e = cl >> 2, k = cl & 3, jj = (k & 1) ? 3 : 1, ip = k >> 1;
   const int nsls = cg.nsls;
   const float4 *cs = reinterpret_cast<const float4 *>(cg.consts + (int64_t)g.slot0 * 48) + cl;
-  const float4 c0 = __ldg(cs), c1 = __ldg(cs + nl), c2 = __ldg(cs + 2 * nl);
+  const float4 *cst = STAGED ? reinterpret_cast<const float4 *>(sc + kScConst) + cl : cs;
+  const int crow = STAGED ? kCgLanes : nl;
+  if (STAGED) cp_async_wait_all();
+  const float4 c0 = cst[0], c1 = cst[crow], c2 = cst[2 * crow];
+  const float2 *ss = reinterpret_cast<const float2 *>(sc + kScState) + cl;
   const float dmu = c0.x, dka = c0.y, yl = c0.z, vse = c0.w, vsx = c1.x, vze = c1.y, vzx = c1.z;
   float *sbase = cg.state + (int64_t)g.slot0 * 4 * cg_state_floats(nsls);
   float2 *st = reinterpret_cast<float2 *>(sbase) + cl;
@@ -356,22 +397,24 @@ __device__ __forceinline__ void cg_point(const CgArgs &cg, const float *xw, floa
     float dv[6];
 #pragma unroll
     for (int w = 0; w < 3; ++w) {
-      const float2 t = st[(3 * nsls + w) * nl];
+      const float2 t = STAGED ? ss[(3 * kCgBatch + w) * kCgLanes] : st[(3 * nsls + w) * nl];
       dv[2 * w] = t.x;
       dv[2 * w + 1] = t.y;
     }
-    const float tk = *trp;
+    const float tk = STAGED ? sc[kScTr + cl] : *trp;
     const bool store = mine && lane < nl;
-    for (int q0 = 0; q0 < nsls; q0 += kCgBatch) {
+    constexpr int kB = STAGED ? 1 : kCgBatch;
+    for (int q0 = 0; q0 < nsls; q0 += kB) {
       // the batch's loads are issued together, before its stores
-      float2 R[kCgBatch][3];
+      float2 R[kB][3];
 #pragma unroll
-      for (int b = 0; b < kCgBatch; ++b)
+      for (int b = 0; b < kB; ++b)
         if (q0 + b < nsls)
 #pragma unroll
-          for (int w = 0; w < 3; ++w) R[b][w] = st[(3 * (q0 + b) + w) * nl];
+          for (int w = 0; w < 3; ++w)
+            R[b][w] = STAGED && q0 < kCgBatch ? ss[(3 * q0 + w) * kCgLanes] : st[(3 * (q0 + b) + w) * nl];
 #pragma unroll
-      for (int b = 0; b < kCgBatch; ++b) {
+      for (int b = 0; b < kB; ++b) {
         const int q = q0 + b;
         if (q >= nsls) break;
         const float tm = __ldg(tmu + q), tm1 = __ldg(tmu + kMaxSls + q);
@@ -440,7 +483,6 @@ __device__ __forceinline__ void cg_point(const CgArgs &cg, const float *xw, floa
     }
   }
 }
-constexpr int kScFloats = 9 * kCgLanes;  // per warp
 
 // the columns j = 1, 3 leave the derivatives and displacements of their two
 // cg points for cg_point (18 of the lane's 20 exchange floats)
@@ -509,7 +551,7 @@ __device__ __forceinline__ void col_stiffness(const SpecDev &sp, const float (&e
   if (ANEL) {
     if (MODE == MODE_NEWMARK) cg_put<POLE, NC>(xw, lane, j, X, E, u);
     __syncwarp();
-    cg_point<POLE, MODE == MODE_NEWMARK>(cg, xw, sc, g, lane, mine_cg);
+    cg_point<POLE, MODE == MODE_NEWMARK, MODE == MODE_NEWMARK>(cg, xw, sc, g, lane, mine_cg);
     rows(1, (OFF + NT - 1) / 8);
     __syncwarp();
   }
@@ -702,7 +744,10 @@ __device__ __forceinline__ void solid_group(const StreamWork &w, const SpecDev &
     if (!ANEL)
 #pragma unroll
       for (int r = 1; r <= (G::kOff + G::NT - 1) / 8; ++r) ldg8(blk + (int64_t)r * 8 * nl, mv[r], pol);
+    constexpr bool staged = ANEL && MODE == MODE_NEWMARK;
+    if (staged) cg_stage_consts(w.cg, sc, g, lane);
     const bool stopped = wait();
+    if (staged) cg_stage_state(w.cg, sc, g, lane);
     float u[NC][5], f[NC][5];
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
@@ -1159,10 +1204,11 @@ struct SolidPoint {
 
 // An inner GLL point of an element of a scattered solid (nine per element, 9/16
 // of the points): one copy, whose place follows from the point's number
-// 9 slot + 3 (j - 1) + i - 1, so no index is read: steps of 353 000 points took
-// 25.1 us with all points through the lists below and take 24.8 (compensated),
-// 15.4 / 13.9 without; with cg4 on 2.2 million points 49.5 / 47.6.  (Finished by
-// the element pass itself they cost more: its chain is the longer one.)
+// 9 slot + 3 (j - 1) + i - 1, so no index is read: steps of 305 000 points took
+// 25.1 us with all points through the lists below and take 24.9 (quadrupole,
+// compensated), 24.0 / 21.6 (dipole); with cg4 on 99 450 elements 137.4 /
+// 132.1.  (Finished by the element pass itself they cost more: its chain is the
+// longer one.)
 template <int POLE, int MODE, bool KAHAN>
 __device__ __forceinline__ void inner_point(const StreamWork &w, int32_t g) {
   using S = SolidPoint<POLE, MODE, KAHAN>;
@@ -1465,12 +1511,12 @@ template <int POLE, int MODE, bool ANEL, bool KAHAN, int CTAS, class P>
 __global__ void __launch_bounds__(kGrpThreads, CTAS)
     scatter_kernel(const __grid_constant__ P p, const __grid_constant__ SpecDev sp) {
   __shared__ __align__(16) float xch[kGrpWarps * kXchFloats];
-  __shared__ float scr[ANEL ? kGrpWarps * kScFloats : 1];
+  __shared__ __align__(16) float scr[ANEL ? kGrpWarps * kScFloats : 1];
   elem_cta<POLE, false, MODE, ANEL, KAHAN>(p, sp, xch, scr, nullptr);
 }
-// The element pass of larger meshes (without coarse-grained attenuation): 3 CTAs per SM took 21.6 ms where 4 took
-// 23.1 (30 steps, quadrupole, 1 048 576 elements); a monopole keeps 4 (18.1 ms
-// against 20.3).
+// The element pass of larger meshes (without coarse-grained attenuation): 3
+// CTAs per SM took 21.7 ms where 4 took 23.1 (32 steps, quadrupole, 786 432
+// solid elements); a monopole keeps 4 (18.1 ms against 20.3).
 template <int POLE, int MODE, bool KAHAN, class P>
 __global__ void __launch_bounds__(kGrpThreads, POLE != POLE_MONO ? 3 : 4)
     patch_kernel(const __grid_constant__ P p, const __grid_constant__ SpecDev sp) {
@@ -1558,7 +1604,7 @@ __global__ void __launch_bounds__(kGrpThreads, 4)
   __syncwarp();
   cg_put<POLE, NC>(xw, lane, j, X, E, u);
   __syncwarp();
-  cg_point<POLE, true>(w.cg, xw, nullptr, g, lane, true);
+  cg_point<POLE, true, false>(w.cg, xw, nullptr, g, lane, true);
 }
 
 }  // namespace axg

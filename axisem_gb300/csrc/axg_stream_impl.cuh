@@ -26,7 +26,7 @@ unsigned blocks(const StreamMany &p) { return (unsigned)p.start[p.n]; }
 // L2 12.9 / 14.0 us on 13 390 elements, from HBM 20.1 / 17.0 on 18 944, 23.9 /
 // 23.6 on 25 802, 32.4 / 33.2 on 32 298 (3 waves either way), 73.2 / 71.3 on
 // 70 528.  Several solves' launches, whose waves fill, keep 4: six solves on
-// 5 664 elements each 9.67 / 9.95 ms for 100 steps.
+// 5 664 and 18 944 elements 9.67 / 9.95 ms for 96 steps.
 template <int POLE, int MODE, bool ANEL, bool KAHAN, class P>
 auto scatter_of(const StreamKernel &k) -> void (*)(P, SpecDev) {
   if constexpr (ANEL) return scatter_kernel<POLE, MODE, ANEL, KAHAN, 3, P>;

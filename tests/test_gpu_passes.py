@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 from axisem_gb300 import _abi, sphere
-from axisem_gb300.mesh import coupled_mesh, gauss_at, gvec_to_elemental, random_gvec, structured_mesh
+from axisem_gb300.mesh import add_attenuation, coupled_mesh, gauss_at, gvec_to_elemental, random_gvec, structured_mesh
 from axisem_gb300.solver import Solver, symplectic_coefficients
 
 pytestmark = pytest.mark.gpu
@@ -32,6 +32,22 @@ def test_group_remainders(gpu_lib, orc, pole, ni, nj, axial):
         f = s.stiffness_assembled(u)
         assert np.array_equal(f, s.stiffness_assembled(u))
     assert rel(f, orc.stiffness_assembled(m, u, np.float64)) <= 1e-5
+
+
+@pytest.mark.parametrize("pole", [0, 1, 2])
+@pytest.mark.parametrize("n_sls", [1, 5, 6, 8])
+def test_memory_variables_staged(gpu_lib, orc, pole, n_sls):
+    """The memory variables of up to five solids are staged in shared memory,
+    further ones read directly; groups of fewer elements at the end."""
+    m = add_attenuation(coupled_mesh(7, 5, 3, pole, niter=30), n_sls=n_sls)
+    t = orc.TimeLoop(m, np.float64)
+    assert t.run(1, m.niter) == 0
+    with Solver(m) as s:
+        s.run(1, m.niter)
+        assert rel(s.receivers(), t.receivers()) <= 1e-4
+        # (the monopole never writes components 4 and 6)
+        mc = [0, 1, 2, 4] if pole == 0 else list(range(6))
+        assert rel(s.get_state(_abi.FIELD_MEMVAR)[:, mc], t.memvar[:, mc]) <= 1e-4
 
 
 @pytest.mark.parametrize("pole", [0, 1, 2])
