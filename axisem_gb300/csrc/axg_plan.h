@@ -11,6 +11,11 @@
 // are added (pre-pass, then colour 0, 1, ...) is fixed: results are
 // bit-reproducible run to run.
 //
+// The no-allocation stiffness runs the plan in that form.  The step's two passes
+// (axg_stream.cuh) take from it the order of elements, patches and sub-rounds;
+// their patches need no colours, since a patch's sums of shared points go to
+// places of its own.
+//
 // The planner is plain C++ with no CUDA dependency so that it can be checked
 // on a machine without a GPU.
 #pragma once

@@ -15,8 +15,8 @@ receiver count and a seismogram duration.  The server
     stream (axg_run_async), so that the solves' kernels overlap on the GPU,
     and polls them (axg_poll); a finished solve returns its seismograms and
     frees its memory, which admits the next request;
-  * or, batched, advances all admitted solves together (axg_batch_*): one
-    launch per colour and kernel class covers every solve's patches, and a
+  * or, batched, advances all admitted solves together (axg_batch_*): an
+    element pass and a point pass per kernel class cover every solve, and a
     step is one CUDA graph replay.  Between chunks finished solves retire and
     waiting ones join (continuous batching at chunk granularity); new solves
     are created while the current chunk runs.

@@ -267,9 +267,9 @@ class Solver:
 
 
 class Batch:
-    """Several solves advanced together (axg_batch_*): one launch per colour
-    and kernel class covers all of them, and the step is replayed from one
-    CUDA graph.  Each solve's results are bit-for-bit those it gets alone.
+    """Several solves advanced together (axg_batch_*): two launches per
+    kernel class cover all of them, and the step is replayed from a CUDA
+    graph.  Each solve's results are bit-for-bit those it gets alone.
     The solvers must stay open while the batch exists."""
 
     def __init__(self, solvers: "list[Solver]"):

@@ -283,7 +283,7 @@ def measure_stiffness(args, pole, ws, rank, local, e2e=True):
     out["roofline"] = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                        "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                        "algorithmic_bytes_per_step": nbytes,
-                       "kernel": f"solid_patch_kernel<{name},force> (all colour launches of one step)"}
+                       "kernel": f"patch_kernel<{name},force> and point_kernel<{name},force> (the two launches of one step)"}
     return out
 
 

@@ -197,7 +197,7 @@ const char *axg_version(void);
 int axg_device_count(void);
 
 /* Copies the mesh, metric terms, source and receiver tables to HBM and builds
- * the element patches, the patch colouring and the point renumbering.
+ * the element order and patches of the step and the point renumbering.
  * Replaces the data hand-over before SOLVER/time_evol_wave.F90:264 (the
  * Fortran module arrays of data_matr / data_mesh / data_source).
  * `*out` is set to a handle (or NULL on failure, with the reason in
@@ -301,13 +301,13 @@ int axg_poll(axg_handle *h, int32_t *done);
 int axg_wait(axg_handle *h);
 
 /* Batches: several solves advanced together, on the same or on different
- * meshes (uneven element counts).  A batch step makes one launch per colour
- * and kernel class for all its solves -- the kernels take a work list of
- * (solve, patch) items -- and is captured once in a CUDA graph that every
- * step replays.  Solves of a batch may differ in pole, precision mode
+ * meshes (uneven element counts).  A batch step makes two launches (an
+ * element pass and a point pass) per kernel class for up to 12 solves -- the
+ * kernels take a list of the solves' work -- and is captured in CUDA graphs
+ * that the steps replay.  Solves of a batch may differ in pole, precision mode
  * (plain or compensated), attenuation (cg4) and time scheme: a symplectic
  * solve's stages run as phases of the batch step (stage i of every solve
- * with more than i stages in one launch per colour and kernel class).  They
+ * with more than i stages in the same launches).  They
  * share the GLL derivative matrices; solves that dump wavefields or
  * checkpoint seismograms run alone.  Each solve's results are bit-for-bit
  * those it gets alone.  The handles must stay open while the batch exists
@@ -399,7 +399,9 @@ typedef struct axg_info {
 int axg_get_info(axg_handle *h, axg_info *info);
 
 /* Per-element patch colour of the solid elements (1-based reference order);
- * for validation of the atomic-free colouring. */
+ * for validation of the atomic-free colouring (axg_stiffness_assembled_noalloc
+ * launches by it; the step's passes take the order of patches and sub-rounds
+ * from the same plan). */
 int axg_get_solid_colouring(axg_handle *h, int32_t *patch_of_elem, int32_t *colour_of_patch,
                             int64_t n_patch_cap);
 
@@ -503,7 +505,7 @@ int axg_set_seismogram_checkpoint(axg_handle *h, int32_t check_it, float *out, i
 int axg_seismogram_checkpoint_samples(axg_handle *h, int32_t *n_samples);
 
 /* Event-timed repeat of axg_stiffness_assembled_device: n launches, returns the
- * average device time in ms of one stiffness+assembly (all colour launches). */
+ * average device time in ms of one stiffness+assembly (its two launches). */
 int axg_time_stiffness(axg_handle *h, int32_t n, float *ms_avg);
 
 /* Debug builds compiled with -DAXG_DEVICE_CHECKS check every device index
