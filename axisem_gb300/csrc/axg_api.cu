@@ -3132,14 +3132,25 @@ int axg_wavefield_dump_layout(axg_handle *h, int32_t *n_solid_fields, int32_t *n
 
 // ------------------------------------------------------------ batches
 
+constexpr int kBatchClasses = 24;  // pole, form of the element pass, attenuation, precision mode
+// Steps per graph of a batch (even: the buffers' roles return).  Six compensated
+// solves of all poles on 50 s and 25 s meshes took 9.52 ms for 96 steps with
+// a graph per step and the classes one after another, and take 8.57 with
+// eight steps per graph and a branch per class.
+constexpr int kBatchSteps = 8;
+
 struct axg_batch {
   std::vector<axg_handle *> hs;
   int device = 0, num_sms = 1;
   SpecDev spec{};
   cudaStream_t stream = nullptr;
-  // one step of every solve, captured with the plain Newmark solves' buffer
-  // roles at parity 0 and at parity 1 (trade_buffers); steps alternate them
-  cudaGraphExec_t graph[2] = {};
+  // one step of every solve, captured with the Newmark solves' buffer roles at
+  // parity 0 and at parity 1 (trade_buffers), and kBatchSteps steps from
+  // parity 0; steps alternate the parities
+  cudaGraphExec_t graph[2] = {}, graph_many = nullptr;
+  // the captures' branches, one per class of Newmark solves
+  cudaStream_t branch[kBatchClasses] = {};
+  cudaEvent_t ev_branch = nullptr;
   cudaEvent_t ev_done = nullptr;
   bool pending = false;
   int64_t launches_per_step = 0;
@@ -3201,22 +3212,26 @@ void stage_states(axg_handle *h, int stage, StateArgs &ss, StateArgs &fs) {
   }
 }
 
+int batch_class(const axg_handle *h) {
+  return h->pole * 8 + (h->os.patched ? 4 : 0) + (h->anel ? 2 : 0) + (h->kahan ? 1 : 0);
+}
+
 // One phase of the solves taking part in it, as enqueue_step (a stage of
 // enqueue_step_symplectic) queues it for one: launch q of every solve of a
 // class (pole, form of the element pass, precision mode, attenuation) in one
-// launch.
+// launch.  The classes of a Newmark step have branches of their own: nothing
+// of theirs depends on another class.
 int64_t enqueue_batch_phase(axg_batch *b, int stage, cudaStream_t s) {
   const int mode = stage < 0 ? MODE_NEWMARK : MODE_SYMPLECTIC;
   int64_t nl = 0;
-  for (int cls = 0; cls < 24; ++cls) {
+  for (int cls = 0; cls < kBatchClasses; ++cls) {
     const int pole = cls / 8;
+    const cudaStream_t cs = stage < 0 && b->branch[cls] ? b->branch[cls] : s;
     const bool kahan = cls & 1, anel = (cls & 2) != 0, patched = (cls & 4) != 0;
     // per launch of the class: its kind and the solves' work
     std::vector<std::pair<int, std::vector<StreamWork>>> seq;
     for (axg_handle *h : b->hs) {
-      if (!in_stage(h, stage) || h->pole != pole || h->kahan != kahan || h->anel != anel ||
-          h->os.patched != patched)
-        continue;
+      if (!in_stage(h, stage) || batch_class(h) != cls) continue;
       StateArgs ss, fs;
       stage_states(h, stage, ss, fs);
       size_t q = 0;
@@ -3236,9 +3251,9 @@ int64_t enqueue_batch_phase(axg_batch *b, int stage, cudaStream_t s) {
           ++m.n;
         }
         const StreamKernel k{l.first, mode, patched, anel, kahan};
-        if (pole == AXG_MONOPOLE) stream_launch<POLE_MONO>(k, m, b->spec, s);
-        else if (pole == AXG_DIPOLE) stream_launch<POLE_DI>(k, m, b->spec, s);
-        else stream_launch<POLE_QUAD>(k, m, b->spec, s);
+        if (pole == AXG_MONOPOLE) stream_launch<POLE_MONO>(k, m, b->spec, cs);
+        else if (pole == AXG_DIPOLE) stream_launch<POLE_DI>(k, m, b->spec, cs);
+        else stream_launch<POLE_QUAD>(k, m, b->spec, cs);
         ++nl;
       }
   }
@@ -3288,6 +3303,32 @@ __global__ void set_iters_kernel(const __grid_constant__ IterSet a) {
   if ((int)threadIdx.x < a.n) *a.ctr[threadIdx.x] = a.first[threadIdx.x];
 }
 
+// `steps` steps of every solve into a graph, from the buffers' current roles
+// (which it trades for each step; a failed capture leaves them as they were)
+int batch_capture(axg_batch *b, int steps, cudaGraphExec_t *exec) {
+  cudaGraph_t g;
+  BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+  cudaEventRecord(b->ev_branch, b->stream);
+  for (cudaStream_t br : b->branch)
+    if (br) cudaStreamWaitEvent(br, b->ev_branch, 0);
+  for (int q = 0; q < steps; ++q) b->launches_per_step = enqueue_batch_step(b, b->stream);
+  for (cudaStream_t br : b->branch)
+    if (br) {
+      cudaEventRecord(b->ev_branch, br);
+      cudaStreamWaitEvent(b->stream, b->ev_branch, 0);
+    }
+  const cudaError_t le = cudaGetLastError();
+  const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
+  cudaError_t e = le != cudaSuccess ? le : ce;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
+  if (ce == cudaSuccess) cudaGraphDestroy(g);
+  if (e == cudaSuccess) return AXG_OK;
+  if (steps & 1)
+    for (axg_handle *h : b->hs) trade_buffers(h);
+  return bfail(b, e == cudaErrorMemoryAllocation ? AXG_ERR_OOM : AXG_ERR_CUDA,
+               fmt("batch step capture: %s", cudaGetErrorString(e)));
+}
+
 int batch_create_impl(axg_batch *b, axg_handle *const *hs, int32_t n) {
   if (!hs || n < 1) return bfail(b, AXG_ERR_BAD_ARG, "axg_batch_create: no handles");
   for (int k = 0; k < n; ++k) {
@@ -3319,25 +3360,23 @@ int batch_create_impl(axg_batch *b, axg_handle *const *hs, int32_t n) {
     BCK(normalize_buffers(h, h->stream));
     BCK(cudaStreamSynchronize(h->stream));
   }
-  // one step, captured once per parity; every step of every run replays one
-  for (int p = 0; p < 2; ++p) {
-    cudaGraph_t g;
-    BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    b->launches_per_step = enqueue_batch_step(b, b->stream);  // (trades the buffers: parity p + 1)
-    const cudaError_t le = cudaGetLastError();
-    const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
-    if (le != cudaSuccess || ce != cudaSuccess) {
-      if (ce == cudaSuccess) cudaGraphDestroy(g);
-      if (p == 0)
-        for (axg_handle *h : b->hs) trade_buffers(h);  // back to parity 0
-      return bfail(b, AXG_ERR_CUDA, fmt("batch step capture: %s", cudaGetErrorString(le != cudaSuccess ? le : ce)));
-    }
-    const cudaError_t ie = cudaGraphInstantiate(&b->graph[p], g, 0);
-    cudaGraphDestroy(g);
-    if (ie != cudaSuccess && p == 0)
-      for (axg_handle *h : b->hs) trade_buffers(h);
-    BCK(ie);
+  // a branch per class, where there is more than one
+  BCK(cudaEventCreateWithFlags(&b->ev_branch, cudaEventDisableTiming));
+  bool several = false;
+  for (axg_handle *h : b->hs)
+    several = several || batch_class(h) != batch_class(b->hs[0]) || h->scheme != b->hs[0]->scheme;
+  if (several)
+    for (axg_handle *h : b->hs)
+      if (h->scheme == AXG_SCHEME_NEWMARK2 && !b->branch[batch_class(h)])
+        BCK(cudaStreamCreateWithFlags(&b->branch[batch_class(h)], cudaStreamNonBlocking));
+  // captured once; every step of every run replays one
+  int rc = batch_capture(b, kBatchSteps, &b->graph_many);
+  for (int p = 0; p < 2 && !rc; ++p) {
+    rc = batch_capture(b, 1, &b->graph[p]);
+    if (rc && p == 1)
+      for (axg_handle *h : b->hs) trade_buffers(h);  // back to parity 0
   }
+  if (rc) return rc;
   return AXG_OK;
 }
 
@@ -3345,6 +3384,10 @@ void batch_release(axg_batch *b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   for (cudaGraphExec_t g : b->graph)
     if (g) cudaGraphExecDestroy(g);
+  if (b->graph_many) cudaGraphExecDestroy(b->graph_many);
+  for (cudaStream_t br : b->branch)
+    if (br) cudaStreamDestroy(br);
+  if (b->ev_branch) cudaEventDestroy(b->ev_branch);
   if (b->ev_done) cudaEventDestroy(b->ev_done);
   if (b->stream) cudaStreamDestroy(b->stream);
 }
@@ -3406,7 +3449,9 @@ int axg_batch_run_async(axg_batch *b, const int32_t *first_iters, int32_t n_iter
     set_iters_kernel<<<1, kMaxBatch, 0, b->stream>>>(a);
   }
   BCK(cudaGetLastError());
-  for (int32_t q = 0; q < n_iter; ++q) {
+  int32_t q = 0;
+  for (; q + kBatchSteps <= n_iter; q += kBatchSteps) BCK(cudaGraphLaunch(b->graph_many, b->stream));
+  for (; q < n_iter; ++q) {
     BCK(cudaGraphLaunch(b->graph[q & 1], b->stream));
     for (axg_handle *h : b->hs) trade_buffers(h);
   }
