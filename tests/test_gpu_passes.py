@@ -13,7 +13,7 @@ import pytest
 
 from axisem_gb300 import _abi, sphere
 from axisem_gb300.mesh import add_attenuation, coupled_mesh, gauss_at, gvec_to_elemental, random_gvec, structured_mesh
-from axisem_gb300.solver import Solver, symplectic_coefficients
+from axisem_gb300.solver import Batch, Solver, symplectic_coefficients
 
 pytestmark = pytest.mark.gpu
 
@@ -160,3 +160,26 @@ def test_mass_pairs_against_fp64_masses(gpu_lib, pole, seconds):
     for a, b in list(zip(*recs))[:1 if seconds < 100 else 2]:   # (the wave reaches the fluid later)
         assert np.linalg.norm(b) > 0
         assert rel(a, b) <= m.niter * 2.0 ** -24
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_batch_beyond_l2(gpu_lib, shared):
+    """Meshes whose blocks exceed L2 only together, with 13 steps (a graph of
+    several and single ones): bit for bit each solve's own run."""
+    n = 13
+    ms = [coupled_mesh(110, 85, 7, p, niter=n, num_rec=4, src_row=9) for p in (1, 2)]
+    ms.append(ms[1] if shared else coupled_mesh(31, 17, 5, 2, niter=n, num_rec=4, src_row=4))
+    alone = []
+    for m in ms:
+        with Solver(m) as s:
+            s.run(1, n)
+            alone.append((s.receivers(), s.get_state(_abi.FIELD_DISP)))
+    solvers = [Solver(m) for m in ms[:2]]
+    solvers.append(Solver(ms[2], share_with=solvers[1]) if shared else Solver(ms[2]))
+    with Batch(solvers) as b:
+        b.run([1] * 3, n)
+    for s, (rec, disp) in zip(solvers, alone):
+        assert np.array_equal(s.receivers(), rec) and np.array_equal(s.get_state(_abi.FIELD_DISP), disp)
+        assert np.abs(disp).max() > 0
+    for s in reversed(solvers):
+        s.close()
