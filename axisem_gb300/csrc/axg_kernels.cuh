@@ -78,7 +78,6 @@ enum : int {
 };
 __host__ __device__ constexpr int n_terms(int pole) { return pole == POLE_MONO ? 15 : (pole == POLE_DI ? 24 : 26); }
 __host__ __device__ constexpr int n_axial(int pole) { return pole == POLE_MONO ? 3 : (pole == POLE_DI ? 9 : 6); }
-__host__ __device__ constexpr int block_stride(int nt) { return ((nt * 25 + 3) / 4) * 4; }
 // solid element block: nt*25 metric floats, then 25 uint16 patch-local point
 // indices (50 bytes), 2 bytes pad, the int32 element info word; 16-byte multiple
 __host__ __device__ constexpr int solid_idx_off(int nt) { return nt * 25; }      // in floats
