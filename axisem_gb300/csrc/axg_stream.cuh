@@ -234,7 +234,7 @@ __device__ __forceinline__ void xch_put(float *xw, int lane, const float (&v)[NC
     p[q] = t;
   }
 }
-// out[c][i] += sum_k v_k[c][i] coef[k], v_k the values lane e5 + k put
+// out[c][i] = sum_k v_k[c][i] coef[k], v_k the values lane e5 + k put
 template <int NC>
 __device__ __forceinline__ void xch_eta(const float *xw, int e5, const float (&coef)[5], float (&out)[NC][5]) {
 #pragma unroll
@@ -247,29 +247,24 @@ __device__ __forceinline__ void xch_eta(const float *xw, int e5, const float (&c
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int x = 4 * q + r;
-        if (x < 5 * NC) out[x / 5][x % 5] = fmaf(tv[r], coef[k], out[x / 5][x % 5]);
+        if (x < 5 * NC) out[x / 5][x % 5] = k == 0 ? tv[r] * coef[k] : fmaf(tv[r], coef[k], out[x / 5][x % 5]);
       }
     }
   }
 }
-// out[c][i] += sum_k v[c][k] M(k, i) with M(k, i) = g[k + 5 i] (first stage)
+// out[c][i] = sum_k v[c][k] M(k, i) with M(k, i) = g[k + 5 i] (first stage)
 // or g[i + 5 k] (second stage)
 template <int NC, bool SECOND>
 __device__ __forceinline__ void col_xi(const float *g, const float (&v)[NC][5], float (&out)[NC][5]) {
 #pragma unroll
   for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int i = 0; i < 5; ++i)
+    for (int i = 0; i < 5; ++i) {
+      float s = g[SECOND ? i : 5 * i] * v[c][0];
 #pragma unroll
-      for (int k = 0; k < 5; ++k) out[c][i] = fmaf(SECOND ? g[i + 5 * k] : g[k + 5 * i], v[c][k], out[c][i]);
-}
-
-template <int NC>
-__device__ __forceinline__ void col_zero(float (&v)[NC][5]) {
-#pragma unroll
-  for (int c = 0; c < NC; ++c)
-#pragma unroll
-    for (int i = 0; i < 5; ++i) v[c][i] = 0.f;
+      for (int k = 1; k < 5; ++k) s = fmaf(SECOND ? g[i + 5 * k] : g[k + 5 * i], v[c][k], s);
+      out[c][i] = s;
+    }
 }
 
 // component c of a group array is the axis-masked one of the pole (group
@@ -541,8 +536,6 @@ __device__ __forceinline__ void col_stiffness(const SpecDev &sp, const float (&e
     }
   };
   float X[NC][5], E[NC][5];
-  col_zero(X);
-  col_zero(E);
   xch_put<NC>(xw, lane, u);
   __syncwarp();
   col_xi<NC, false>(gxi, u, X);
@@ -635,11 +628,25 @@ __device__ __forceinline__ void col_stiffness(const SpecDev &sp, const float (&e
       }
     }
   }
-  // second stage: f += mxm(G, S1) + mxm(S2, G2T), S1 in X
+  // second stage: f and mxm(G, S1) and mxm(S2, G2T), S1 in X, each sum formed
+  // apart and added in the reference's order.  Ten terms in a chain on top of f
+  // round at f's magnitude (stiffness errors against FP64 of 6.7e-8, these
+  // 6.3e-8, quadrupole), and f + (first + second) has 6.6e-8.  The additions
+  // cost 4 % of a quadrupole's step from HBM (19.7 to 20.6 us on 18 944 elements)
+  // and of an attenuated dipole's (131 to 136 on 99 450); others take as long.
   xch_put<NC>(xw, lane, S2);
   __syncwarp();
-  col_xi<NC, true>(gxi, X, f);
-  xch_eta<NC>(xw, e5, seta, f);
+  float Y[NC][5];
+  col_xi<NC, true>(gxi, X, Y);
+  xch_eta<NC>(xw, e5, seta, E);
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      if (POLE == POLE_DI ? c == 0 : POLE == POLE_MONO && c == 1) f[c][i] = Y[c][i] + E[c][i];  // (no local part)
+      else if (POLE == POLE_DI) f[c][i] = Y[c][i] + E[c][i] + f[c][i];
+      else f[c][i] = f[c][i] + Y[c][i] + E[c][i];
+    }
   __syncwarp();
   if (AX) {
     auto w = [&](int q) { return m0[5 * q + j]; };
@@ -895,15 +902,12 @@ __device__ __forceinline__ void fluid_group(const StreamWork &w, const SpecDev &
   }
   if (NONMONO && ax) chi[0][0] = 0.f;  // apply_axis_mask_scal
   float X[1][5], E[1][5], f[1][5];
-  col_zero(X);
-  col_zero(E);
   xch_put<1>(xw, lane, chi);
   __syncwarp();
   xch_eta<1>(xw, e5, eta, E);
-  if (axm != kFull) col_xi<1, false>(sp.g2, chi, X);
+  col_xi<1, false>(sp.g2, chi, X);
   if (axm) {
     float Y[1][5];
-    col_zero(Y);
     col_xi<1, false>(sp.g1, chi, Y);
 #pragma unroll
     for (int i = 0; i < 5; ++i)
@@ -917,22 +921,23 @@ __device__ __forceinline__ void fluid_group(const StreamWork &w, const SpecDev &
     const float x1 = X[0][i], x2 = E[0][i];
     X[0][i] = m[0] * x2 + m[1] * x1;
     S2[0][i] = m[0] * x1 + m[2] * x2;
-    f[0][i] = NONMONO ? m[NT - 1] * chi[0][i] : 0.f;
   }
   xch_put<1>(xw, lane, S2);
   __syncwarp();
+  col_xi<1, true>(sp.g2, X, f);
   if (axm) {
-    float a[1][5], b[1][5];
-    col_zero(a);
-    col_zero(b);
-    col_xi<1, true>(sp.g1, X, a);
-    col_xi<1, true>(sp.g2, X, b);
+    float Y[1][5];
+    col_xi<1, true>(sp.g1, X, Y);
 #pragma unroll
-    for (int i = 0; i < 5; ++i) f[0][i] = f[0][i] + (ax ? a[0][i] : b[0][i]);
-  } else {
-    col_xi<1, true>(sp.g2, X, f);
+    for (int i = 0; i < 5; ++i)
+      if (ax) f[0][i] = Y[0][i];
   }
-  xch_eta<1>(xw, e5, seta, f);
+  xch_eta<1>(xw, e5, seta, E);
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    f[0][i] = f[0][i] + E[0][i];
+    if (NONMONO) f[0][i] = fmaf(mv[5 + i * NT + NT - 1], chi[0][i], f[0][i]);
+  }
   if (ax || d.srcfl) {
     const int32_t info = __ldg(d.elinfo + slot);
     int axslot = (info & 0xFFFFFF) - 1;
@@ -1588,9 +1593,6 @@ __global__ void __launch_bounds__(kGrpThreads, 4)
       if (i == 0 && ax && col_masked<POLE>(c)) u[c][i] = 0.f;
     }
   }
-  col_zero(X);
-  col_zero(Y);
-  col_zero(E);
   xch_put<NC>(xw, lane, u);
   __syncwarp();
   col_xi<NC, false>(sp.g2, u, X);
