@@ -248,9 +248,17 @@ __device__ __forceinline__ float drift_comp(float d, float v, const StateArgs &s
 // of an ulp from a tie.  FP64 runs at 1/64 of the FP32 rate here: on 305 000
 // points of three components a compensated step took 27.6 us with FP64
 // products and took 25.1 with pairs; errors against FP64 are alike (2.5e-7).
+// The product's error term is 2^-24 of it and flushed to zero below 2^-126:
+// small products are formed 2^60 times larger (|x| is below 2^30 then, unless
+// the mass is zero).  One that is infinite or no number stays what it is.  (No
+// measurable cost: 4.02 ms for 200 steps of 18 944 elements with and without.)
 __device__ __forceinline__ float mul_pair(float2 m, float x) {
-  const float p = __fmul_rn(m.x, x);
-  return __fadd_rn(p, fmaf(m.y, x, fmaf(m.x, x, -p)));
+  float p = __fmul_rn(m.x, x);
+  const bool small = fabsf(p) < 0x1p-60f && fabsf(x) < 0x1p60f;
+  if (small) x = x * 0x1p60f;
+  if (small) p = __fmul_rn(m.x, x);
+  const float r = __fadd_rn(p, fmaf(m.y, x, fmaf(m.x, x, -p)));
+  return !(fabsf(p) <= 3.402823466e38f) ? p : small ? r * 0x1p-60f : r;
 }
 
 // X(i,j) = sum_k c[k] * v(k,j)   (v(k,j) held by lane k + 5 j)
