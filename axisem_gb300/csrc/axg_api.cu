@@ -161,7 +161,7 @@ struct axg_handle {
   double *inv_mass_s_dp = nullptr, *inv_mass_f_dp = nullptr, *src_val_dp_d = nullptr;
   float2 *inv_mass_s_pair = nullptr, *inv_mass_f_pair = nullptr;  // the same masses, where FP32 pairs hold them
   float *stf = nullptr, *rec = nullptr;
-  int32_t *iter = nullptr, *blowup = nullptr, *rec_gidx_d = nullptr;
+  int32_t *ctl = nullptr, *rec_gidx_d = nullptr;  // ctl: CTL_*
   int32_t *src_gidx_d = nullptr;
   std::vector<int32_t> src_patches;  // patches (scattered: element slots) that own source points, at most 8
   float *src_val_d = nullptr;
@@ -184,7 +184,6 @@ struct axg_handle {
   bool pending = false;
   int num_sms = 1;
   int elem_ctas_force = 1, elem_ctas_step = 1;  // resident CTAs per SM of the element pass
-  int32_t *errw = nullptr, *iter_p = nullptr;
   std::string err = "no error";
   int64_t kernels_per_step = 0, kernels_per_force = 0;
   // time scheme: 0 Newmark (newmark2), else a symplectic scheme of nstages stages
@@ -873,9 +872,10 @@ StateArgs solid_state(axg_handle *h) {
   s.inv_mass_dp = h->kahan ? h->inv_mass_s_dp : nullptr;
   s.gamma = h->gamma_s;
   s.stf = h->stf;
-  s.iter = h->iter;
-  s.blowup = h->blowup;
-  s.err = h->errw;
+  s.iter = h->ctl + CTL_ITER;
+  s.blowup = h->ctl + CTL_BLOWUP;
+  s.stop = h->ctl + CTL_STOP;
+  s.err = h->ctl + CTL_ERR;
   s.thresh = (float)(10.0 * std::fabs(h->magnitude));
   split(h->dt, s.dt, s.dt_lo);
   split(0.5 * h->dt, s.hdt, s.hdt_lo);
@@ -926,7 +926,7 @@ cudaError_t refresh_predicted(axg_handle *h, cudaStream_t s) {
 }
 
 RecWork rec_work(axg_handle *h, const StateArgs &ss) {
-  return RecWork{ss, h->rec_gidx_d, h->num_rec, h->seis_it, h->pole, h->nseismo, h->rec, h->iter};
+  return RecWork{ss, h->rec_gidx_d, h->num_rec, h->seis_it, h->pole, h->nseismo, h->rec, h->ctl};
 }
 
 template <int POLE>
@@ -1017,7 +1017,7 @@ StreamWork stream_work(axg_handle *h, int mode, const StateArgs &ss, const State
   w.solid = ss;
   w.axmask = h->ds.axmask;
   w.cg = h->cg;
-  w.iter_p = h->iter_p;
+  w.ctl = h->ctl;
   w.p0 = (int32_t)h->os.n_own;
   if (streamed(h)) w.prefetch = (mode == MODE_FORCE ? h->elem_ctas_force : h->elem_ctas_step) * h->num_sms;
   if (mode == MODE_FORCE) return w;
@@ -1080,8 +1080,10 @@ template <int POLE>
 void launch_anel_full_pole(axg_handle *h, cudaStream_t s, bool update) {
   const FullAnelArgs fa{h->an, h->fx, h->slot_gidx, h->slot_axial, h->nel_s};
   const unsigned g = (unsigned)std::min<int64_t>((h->nel_s + kWarps - 1) / kWarps, 16 * (int64_t)h->num_sms);
-  if (update) launch_pdl(anel_full_kernel<POLE, true>, g, kThreads, 0, s, fa, solid_state(h), h->spec);
-  else anel_full_kernel<POLE, false><<<g, kThreads, 0, s>>>(fa, solid_state(h), h->spec);
+  StateArgs st = solid_state(h);
+  if (update) st.stop = h->ctl + CTL_STOP_P;  // (it belongs to the step whose point pass has just set CTL_STOP)
+  if (update) launch_pdl(anel_full_kernel<POLE, true>, g, kThreads, 0, s, fa, st, h->spec);
+  else anel_full_kernel<POLE, false><<<g, kThreads, 0, s>>>(fa, st, h->spec);
 }
 void launch_anel_full(axg_handle *h, cudaStream_t s, bool update) {
   if (h->pole == AXG_MONOPOLE) launch_anel_full_pole<POLE_MONO>(h, s, update);
@@ -1117,7 +1119,6 @@ void symplectic_stage_states(axg_handle *h, int i, StateArgs &ss, StateArgs &fs)
   split(h->sym_cd[i], ss.dt, ss.dt_lo);
   split(h->sym_cv[i], ss.kick, ss.kick_lo);
   ss.hdt2 = ss.hdt2_lo = 0.f;  // the coupling's predictor is then the drift u + coefd(i) v
-  ss.stage = fs.stage = 1;
   fs.dt = ss.dt;
   fs.dt_lo = ss.dt_lo;
   fs.kick = ss.kick;
@@ -1813,10 +1814,7 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
   if ((rc = upload(h, &h->rec_gidx_d, h->rec_gidx))) return rc;
   if ((rc = upload(h, &h->src_val_d, src_v))) return rc;
   if (!src_v_dp.empty() && (rc = upload(h, &h->src_val_dp_d, src_v_dp))) return rc;
-  if ((rc = dalloc(h, &h->iter, 4))) return rc;
-  h->blowup = h->iter + 1;
-  h->errw = h->iter + 2;
-  h->iter_p = h->iter + 3;
+  if ((rc = dalloc(h, &h->ctl, kCtlWords))) return rc;
   if ((h->anel || h->anel_full) && (rc = build_anel(h, d, !share))) return rc;
   if ((rc = prepare_kernels(h))) return rc;
   count_launches(h);
@@ -2163,7 +2161,7 @@ int axg_reset(axg_handle *h) {
   h->ckpt.queued = h->ckpt.done = 0;
   // the iter-0 seismogram sample (dump_stuff(0,...)) is the zero wavefield
   CK(cudaMemsetAsync(h->rec, 0, (size_t)h->nseismo * 3 * std::max(h->num_rec, 1) * sizeof(float), h->stream));
-  CK(cudaMemsetAsync(h->iter, 0, 4 * sizeof(int32_t), h->stream));
+  CK(cudaMemsetAsync(h->ctl, 0, kCtlWords * sizeof(int32_t), h->stream));
   if (h->anel_full)
     CK(cudaMemsetAsync(h->an.state, 0, (size_t)h->nel_s * h->an.state_stride * sizeof(float), h->stream));
   if (h->anel) CK(cudaMemsetAsync(h->cg.state, 0, (size_t)cg_floats(h) * sizeof(float), h->stream));
@@ -2187,7 +2185,7 @@ int axg_run(axg_handle *h, int32_t first_iter, int32_t n_iter) {
     CK(cudaHostAlloc((void **)&h->run_flags, 4 * sizeof(int32_t), cudaHostAllocDefault));
     for (cudaEvent_t &e : h->ev_flags) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
-  CK(cudaMemcpyAsync(h->iter, &first_iter, sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->ctl + CTL_ITER, &first_iter, sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
   CK(refresh_predicted(h, h->stream));
   // Graph q + 1 is queued before the flags of graph q are waited for, so that
   // the device does not idle while the host polls (a stopped solve's kernels
@@ -2212,7 +2210,8 @@ int axg_run(axg_handle *h, int32_t first_iter, int32_t n_iter) {
       CK(cudaGetLastError());
     }
     done += k;
-    CK(cudaMemcpyAsync(h->run_flags + 2 * (q & 1), h->blowup, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(h->run_flags + 2 * (q & 1), h->ctl + CTL_BLOWUP, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                       h->stream));
     CK(cudaEventRecord(h->ev_flags[q & 1], h->stream));
     if (q > 0) rc = poll(q - 1);
   }
@@ -2228,7 +2227,7 @@ namespace {
 // reads the device flags after the handle's queued work completed
 int check_flags(axg_handle *h) {
   int32_t flags[2] = {0, 0};
-  CK(cudaMemcpyAsync(flags, h->blowup, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(flags, h->ctl + CTL_BLOWUP, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   if (flags[1] != 0) return fail(h, AXG_ERR_TIMEOUT, "a bounded device wait on a bulk copy gave up");
   if (flags[0] != 0)
@@ -2453,7 +2452,7 @@ int axg_run_async(axg_handle *h, int32_t first_iter, int32_t n_iter) {
   }
   // the kernels of a step after a blow-up return at once, so all steps can
   // be queued without a check in between
-  CK(cudaMemcpyAsync(h->iter, &first_iter, sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(h->ctl + CTL_ITER, &first_iter, sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
   CK(refresh_predicted(h, h->stream));
   for (int32_t done = 0; done < n_iter;) {
     const int32_t it = first_iter + done;
@@ -2542,7 +2541,7 @@ int axg_get_receivers(axg_handle *h, float *out, int32_t cap, int32_t *nseismo_o
   std::vector<float> buf((size_t)h->nseismo * 3 * std::max(h->num_rec, 1));
   CK(cudaMemcpyAsync(buf.data(), h->rec, buf.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
   int32_t it = 0;
-  CK(cudaMemcpyAsync(&it, h->iter, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(&it, h->ctl + CTL_ITER, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   for (int r = 0; r < h->num_rec; ++r)
     for (int c = 0; c < 3; ++c)
@@ -2690,7 +2689,7 @@ int axg_autotune(axg_handle *h, int32_t *chosen) {
   if (h->anel_full) add(h->an.state, (size_t)h->nel_s * h->an.state_stride * sizeof(float));
   if (h->anel) add(h->cg.state, (size_t)cg_floats(h) * sizeof(float));
   add(h->rec, (size_t)h->nseismo * 3 * std::max(h->num_rec, 1) * sizeof(float));
-  add(h->iter, 4 * sizeof(int32_t));
+  add(h->ctl, kCtlWords * sizeof(int32_t));
   size_t total = 0;
   for (auto &p : st) total += (p.second + 255) / 256 * 256;
   char *save = nullptr;
@@ -2715,14 +2714,14 @@ int axg_autotune(axg_handle *h, int32_t *chosen) {
     cudaGraphExec_t g = nullptr;
     if ((rc = build_graph_into(h, k, &g))) break;
     float ms = 0.f;
-    set_counter_kernel<<<1, 1, 0, h->stream>>>(h->iter, 1);
+    set_counter_kernel<<<1, 1, 0, h->stream>>>(h->ctl + CTL_ITER, 1);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaGraphLaunch(g, h->stream);
     int in_run = 1;
     if (e == cudaSuccess) e = cudaEventRecord(h->ev0, h->stream);
     for (int r = 0; r < reps && e == cudaSuccess; ++r) {
       if (in_run == per_run) {
-        set_counter_kernel<<<1, 1, 0, h->stream>>>(h->iter, 1);
+        set_counter_kernel<<<1, 1, 0, h->stream>>>(h->ctl + CTL_ITER, 1);
         e = cudaGetLastError();
         in_run = 0;
       }
@@ -3458,7 +3457,7 @@ int axg_batch_run_async(axg_batch *b, const int32_t *first_iters, int32_t n_iter
     IterSet a{};
     a.n = std::min(kMaxBatch, n - k0);
     for (int q = 0; q < a.n; ++q) {
-      a.ctr[q] = b->hs[k0 + q]->iter;
+      a.ctr[q] = b->hs[k0 + q]->ctl + CTL_ITER;
       a.first[q] = first_iters[k0 + q];
     }
     set_iters_kernel<<<1, kMaxBatch, 0, b->stream>>>(a);

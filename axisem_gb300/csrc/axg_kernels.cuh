@@ -104,6 +104,19 @@ struct DomainArgs {
   int64_t n_patches, n_pts, n_elem, n_m0;   // buffer extents (checked builds)
 };
 
+// A solve's control words (device).  Each of a step's two passes reads what the
+// other writes: the element pass CTL_ITER and CTL_STOP, which the end of the
+// step sets; the point pass the copies that the element pass makes of them.
+enum {
+  CTL_ITER = 0,    // the step counter (1-based iteration of the next step)
+  CTL_BLOWUP = 1,  // first iteration whose displacement blew up (0: none)
+  CTL_ERR = 2,     // AXG_ERR_TIMEOUT when a bounded wait gave up
+  CTL_ITER_P = 3,
+  CTL_STOP = 4,    // CTL_BLOWUP of the steps completed: the solve has stopped
+  CTL_STOP_P = 5,
+  kCtlWords = 8
+};
+
 struct StateArgs {
   float *u[3];              // disp (solid, gvec layout) / chi (fluid: u[0]); plain Newmark: the
                             // buffer the step stores the next step's prediction into
@@ -123,13 +136,13 @@ struct StateArgs {
   const float *stf;         // (niter)
   const int32_t *iter;      // device iteration counter (1-based iter of this step)
   int32_t *blowup;          // first iteration that blew up (0 = none)
+  const int32_t *stop;      // set in the steps after it: they do nothing
   int32_t *err;             // device error word (AXG_ERR_TIMEOUT when a bounded wait gave up)
   float thresh;             // 10 |magnitude|
   // Newmark: deltat, deltat/2, deltat^2/2; symplectic stage: dt = coefd(i) deltat,
   // kick = coefv(i) deltat; each an FP32 pair (value + _lo = the FP64 value)
   float dt, hdt, hdt2, dt_lo, hdt_lo, hdt2_lo;
   float kick, kick_lo;
-  int32_t stage;            // 1 in a symplectic stage (the gathers drift), 0 in a Newmark step
   SrcTable src;
   int64_t nglob;            // extent of the state arrays (checked builds)
   int32_t niter;            // extent of stf
@@ -812,7 +825,7 @@ __global__ void __launch_bounds__(kThreads) anel_full_kernel(const __grid_consta
                                                              SpecDev sp) {
   pdl_wait();
   pdl_trigger();
-  if (*st.blowup) return;
+  if (*st.stop) return;
   const AnelArgs &an = fa.an;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool active = lane < 25;
@@ -1001,7 +1014,7 @@ __global__ void drift_kernel(const __grid_constant__ P p) {
   const StateArgs &solid = p.at(sv).solid;
   const StateArgs &fluid = p.at(sv).fluid;
   const float cd = p.at(sv).cd, cd_lo = p.at(sv).cd_lo;
-  if (*solid.blowup) return;
+  if (*solid.stop) return;
   const int64_t q = it - p.first(sv);
   // u + coefd(nstages+1) v; compensated where the handle keeps compensation
   auto drift = [&](float *u, const float *v, float *cu) {
@@ -1066,7 +1079,7 @@ struct RecWork {
   const int32_t *rec_gidx;
   int32_t num_rec, seis_it, pole, nseismo;
   float *rec;
-  int32_t *iter_ctr;
+  int32_t *ctl;
 };
 template <class P = One<RecWork>>
 __global__ void receivers_kernel(const __grid_constant__ P p) {
@@ -1078,8 +1091,7 @@ __global__ void receivers_kernel(const __grid_constant__ P p) {
   const int32_t *rec_gidx = rw.rec_gidx;
   const int32_t num_rec = rw.num_rec, seis_it = rw.seis_it, pole = rw.pole, nseismo = rw.nseismo;
   float *rec = rw.rec;
-  int32_t *iter_ctr = rw.iter_ctr;
-  const int32_t iter = *iter_ctr;
+  const int32_t iter = rw.ctl[CTL_ITER];
   __syncthreads();
   if (!*solid.blowup && seis_it > 0 && iter % seis_it == 0) {
     const int32_t is = iter / seis_it;
@@ -1100,7 +1112,10 @@ __global__ void receivers_kernel(const __grid_constant__ P p) {
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) *iter_ctr = iter + 1;
+  if (threadIdx.x == 0) {
+    rw.ctl[CTL_STOP] = *solid.blowup;
+    rw.ctl[CTL_ITER] = iter + 1;
+  }
 }
 
 // ------------------------------------------------------------ kernel wavefield dumps
