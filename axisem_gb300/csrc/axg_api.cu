@@ -844,7 +844,7 @@ cudaError_t normalize_buffers(axg_handle *h, cudaStream_t s) {
     std::swap(h->fu, h->fup);
   }
   h->parity = 0;
-  return cudaSuccess;
+  return cudaMemsetAsync(h->ctl + CTL_PARITY, 0, sizeof(int32_t), s);
 }
 
 // an FP64 coefficient as an FP32 pair: hi = its FP32 rounding, lo = the rest
@@ -1018,6 +1018,7 @@ StreamWork stream_work(axg_handle *h, int mode, const StateArgs &ss, const State
   w.axmask = h->ds.axmask;
   w.cg = h->cg;
   w.ctl = h->ctl;
+  w.parity = h->parity ^ 1;
   w.p0 = (int32_t)h->os.n_own;
   if (streamed(h)) w.prefetch = (mode == MODE_FORCE ? h->elem_ctas_force : h->elem_ctas_step) * h->num_sms;
   if (mode == MODE_FORCE) return w;
@@ -2162,6 +2163,8 @@ int axg_reset(axg_handle *h) {
   // the iter-0 seismogram sample (dump_stuff(0,...)) is the zero wavefield
   CK(cudaMemsetAsync(h->rec, 0, (size_t)h->nseismo * 3 * std::max(h->num_rec, 1) * sizeof(float), h->stream));
   CK(cudaMemsetAsync(h->ctl, 0, kCtlWords * sizeof(int32_t), h->stream));
+  const int32_t parity = h->parity;
+  CK(cudaMemcpyAsync(h->ctl + CTL_PARITY, &parity, sizeof parity, cudaMemcpyHostToDevice, h->stream));
   if (h->anel_full)
     CK(cudaMemsetAsync(h->an.state, 0, (size_t)h->nel_s * h->an.state_stride * sizeof(float), h->stream));
   if (h->anel) CK(cudaMemsetAsync(h->cg.state, 0, (size_t)cg_floats(h) * sizeof(float), h->stream));
@@ -2170,6 +2173,22 @@ int axg_reset(axg_handle *h) {
   CK(cudaStreamSynchronize(h->stream));
   return AXG_OK;
 }
+
+}  // extern "C"
+
+namespace {
+// The buffers' roles of a solve that has stopped: the steps queued after the one
+// it stopped in traded them without moving data.
+int settle_stopped(axg_handle *h) {
+  int32_t parity = 0;
+  CK(cudaMemcpyAsync(&parity, h->ctl + CTL_PARITY, sizeof parity, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  if (parity != h->parity) trade_buffers(h);
+  return AXG_OK;
+}
+}  // namespace
+
+extern "C" {
 
 int axg_run(axg_handle *h, int32_t first_iter, int32_t n_iter) {
   if (!h) return fail(nullptr, AXG_ERR_BAD_ARG, "handle is NULL");
@@ -2201,7 +2220,8 @@ int axg_run(axg_handle *h, int32_t first_iter, int32_t n_iter) {
     return AXG_OK;
   };
   int rc = AXG_OK, q = 0;
-  for (int32_t done = 0; done < n_iter && rc == AXG_OK; ++q) {
+  int32_t polled = 0, done = 0;  // steps of the graphs whose flags were read, and of those queued
+  for (; done < n_iter && rc == AXG_OK; ++q) {
     const int k = std::min<int32_t>(h->steps_per_graph, n_iter - done);
     if (k == h->steps_per_graph) {
       if ((rc = launch_graph(h, k, h->graph, h->graph_steps))) break;
@@ -2209,13 +2229,23 @@ int axg_run(axg_handle *h, int32_t first_iter, int32_t n_iter) {
       for (int s = 0; s < k; ++s) enqueue_step(h, h->stream);
       CK(cudaGetLastError());
     }
+    polled = done;
     done += k;
     CK(cudaMemcpyAsync(h->run_flags + 2 * (q & 1), h->ctl + CTL_BLOWUP, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost,
                        h->stream));
     CK(cudaEventRecord(h->ev_flags[q & 1], h->stream));
     if (q > 0) rc = poll(q - 1);
   }
-  if (rc == AXG_OK && q > 0) rc = poll(q - 1);
+  if (rc == AXG_OK && q > 0) {
+    polled = done;
+    rc = poll(q - 1);
+  }
+  if (rc == AXG_ERR_BLOWUP) {
+    // the graph behind the one that stopped counted its steps
+    const int32_t next = first_iter + polled;
+    CK(cudaMemcpyAsync(h->ctl + CTL_ITER, &next, sizeof next, cudaMemcpyHostToDevice, h->stream));
+    if (const int e = settle_stopped(h)) return e;
+  }
   // the run is complete, also where it stopped early
   if (rc != AXG_OK && rc != AXG_ERR_CUDA) CK(cudaStreamSynchronize(h->stream));
   return rc;
@@ -2230,9 +2260,11 @@ int check_flags(axg_handle *h) {
   CK(cudaMemcpyAsync(flags, h->ctl + CTL_BLOWUP, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   if (flags[1] != 0) return fail(h, AXG_ERR_TIMEOUT, "a bounded device wait on a bulk copy gave up");
-  if (flags[0] != 0)
+  if (flags[0] != 0) {
+    if (const int e = settle_stopped(h)) return e;
     return fail(h, AXG_ERR_BLOWUP,
                 fmt("displacements blew up: |disp(1,1,:,:)| > 10 |magnitude| at time step %d", flags[0] + 1));
+  }
   return AXG_OK;
 }
 
@@ -3408,11 +3440,12 @@ void batch_release(axg_batch *b) {
 
 // the solves' flags once the batch's work completed; the first error found
 int batch_flags(axg_batch *b) {
+  int first = AXG_OK;
   for (size_t k = 0; k < b->hs.size(); ++k) {
     const int rc = check_flags(b->hs[k]);
-    if (rc) return bfail(b, rc, fmt("solve %d: %s", (int)k, b->hs[k]->err.c_str()));
+    if (rc && !first) first = bfail(b, rc, fmt("solve %d: %s", (int)k, b->hs[k]->err.c_str()));
   }
-  return AXG_OK;
+  return first;
 }
 
 }  // namespace

@@ -114,6 +114,7 @@ enum {
   CTL_ITER_P = 3,
   CTL_STOP = 4,    // CTL_BLOWUP of the steps completed: the solve has stopped
   CTL_STOP_P = 5,
+  CTL_PARITY = 6,  // roles of the displacement buffers after the last step that was not skipped
   kCtlWords = 8
 };
 
@@ -1040,7 +1041,7 @@ __global__ void drift_kernel(const __grid_constant__ P p) {
 // the step leaves them in its state.
 static __global__ void predict_kernel(StateArgs st, const uint8_t *axmask) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= st.nglob) return;
+  if (q >= st.nglob || *st.stop) return;
   const uint32_t m = axmask ? axmask[q] : 0u;
   for (int c = 0; c < 3; ++c) {
     if (!st.up[c]) continue;

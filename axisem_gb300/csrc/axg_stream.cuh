@@ -163,6 +163,7 @@ struct StreamWork {
   int32_t nb_se, nb_fe, nb_cp, nb_si, nb_sp, nb_fp, nb_rec;  // CTAs per role
   int32_t prefetch;         // element pass: CTAs ahead whose blocks are prefetched into L2 (0: none)
   int32_t *ctl;             // the solve's control words (CTL_*)
+  int32_t parity;           // CTL_PARITY after a Newmark step
   const int32_t *memvar_gidx;  // memvar_kernel: each element slot's 25 points
   RecWork rec;
 };
@@ -1489,6 +1490,7 @@ __device__ __forceinline__ void stream_receivers(const StreamWork &w) {
       }
   }
   if (threadIdx.x == 0) {
+    if (!w.ctl[CTL_STOP_P]) w.ctl[CTL_PARITY] = w.parity;
     w.ctl[CTL_STOP] = *s.blowup;
     w.ctl[CTL_ITER] = iter + 1;
   }

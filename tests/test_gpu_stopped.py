@@ -2,6 +2,7 @@
 step forms; the reference completes that step and stops before the next one
 (runtime_info, SOLVER/time_evol_wave.F90:998-1056).  The step is the same bits as
 without the guard, and the steps queued behind it do nothing."""
+import ctypes as C
 import re
 import time
 
@@ -10,7 +11,7 @@ import pytest
 
 from axisem_gb300 import _abi
 from axisem_gb300.mesh import add_attenuation, coupled_mesh, gauss_at, random_gvec
-from axisem_gb300.solver import AxgError, Solver, symplectic_coefficients
+from axisem_gb300.solver import AxgError, Batch, Solver, symplectic_coefficients
 
 pytestmark = pytest.mark.gpu
 
@@ -102,3 +103,53 @@ def test_steps_after_a_blowup_cost_little(gpu_lib, size, pole, mode):
                 best = min(best, time.perf_counter() - t0)
             took.append(best)
     assert took[1] < 0.5 * took[0], took
+
+
+@pytest.mark.parametrize("size,pole,mode,seed", [(SMALL, 0, "plain", 5), (SMALL, 0, "plain", None), (SMALL, 2, "comp", 5),
+                                                 (SMALL, 1, "cg4", None), (SMALL, 1, "symplec4", 5), (PATCHED, 1, "comp", 5)])
+def test_state_after_a_blowup_whatever_was_queued(gpu_lib, size, pole, mode, seed):
+    """The displacement buffers trade roles every step; those of the steps queued
+    behind a blow-up move nothing.  The state is that of the step that blew up,
+    however many follow it and however they were queued; axg_run counts the steps
+    of the graphs up to the one that stopped (16 each)."""
+    m = _mesh(size, pole, mode, 1e-20)
+    u = None if seed is None else random_gvec(m, seed=seed)
+    if u is not None and pole == 0:
+        u[:, 1] = 0.0
+    with _solver(m, mode, u) as s:
+        k = _blown(lambda: s.run(1, NITER))
+    with _solver(_mesh(size, pole, mode), mode, u) as s:
+        s.run(1, k)
+        want = _state(s, mode)
+
+    def samples(s):
+        n = C.c_int32()
+        out = np.zeros((s.nseismo, 3, m.num_rec), np.float32, order="F")
+        assert gpu_lib.axg_get_receivers(s.h, out.ctypes.data_as(C.POINTER(C.c_float)), s.nseismo, C.byref(n)) == 0
+        return n.value
+
+    def run(s, n):
+        assert _blown(lambda: s.run(1, n)) == k
+        assert samples(s) == min(n, 16) + 1   # (and iteration 0)
+
+    def run_async(s, n):
+        s.run_async(1, n)
+        assert _blown(s.wait) == k
+        assert samples(s) == n + 1
+
+    def in_chunks(s, n):
+        s.run_async(1, n)
+        s.run_async(n + 1, 3)
+        assert _blown(s.wait) == k
+
+    def batch(s, n):
+        with Batch([s]) as b:
+            assert _blown(lambda: b.run([1], n)) == k
+
+    for how in (run, run_async, in_chunks, batch):
+        for n in (k, k + 1, 16, 17, 24, 33):
+            with _solver(m, mode, u) as s:
+                how(s, n)
+                got = _state(s, mode)
+            for f in want:
+                assert np.array_equal(got[f], want[f]), (how.__name__, n, f)
