@@ -205,11 +205,22 @@ class Server:
         return self.meshes[req.key]
 
     def _estimate(self, req: Request) -> int:
+        """Device bytes admitting `req` takes: the solve's own buffers and, if
+        its mesh is not resident, the mesh with the solve that holds it."""
         t = template(req.period, req.pole)
-        nglob = t.nglob_solid + t.nglob_fluid
-        need = nglob * 4 * 4 * 3 + 4 * req.niter * 3 * req.n_rec + (1 << 20)   # wavefields, seismograms
+        nc = 2 if req.pole == _abi.MONOPOLE else 3
+        per_point = 9 if self.compensated else 6   # five fields, three compensations, point tables
+        # the wavefields and the element contributions (columns of 12 or 16 floats, fluid 8)
+        solve = 4 * per_point * (nc * t.nglob_solid + t.nglob_fluid)
+        solve += 20 * ((12 if req.pole == _abi.MONOPOLE else 16) * t.nel_solid + 8 * t.nel_fluid)
+        seis_it = max(1, int(round(req.period / 8.0 / t.deltat)))
+        need = solve + 4 * req.niter + 4 * 3 * req.n_rec * (req.niter // seis_it + 1) + (1 << 20)
         if req.key not in self.meshes:
-            need += 4 * need   # a mesh is a few times its wavefields
+            # metric terms and index words of every point, then masses, coupling
+            # and the points' lists of contributions
+            terms = len(_abi.SOLID_TERMS_USED[req.pole])
+            need += solve + 100 * ((terms + 3) * t.nel_solid + 8 * t.nel_fluid)
+            need += 20 * (t.nglob_solid + t.nglob_fluid)
         return need
 
     def preload(self, keys):
