@@ -35,7 +35,7 @@ namespace axg {
 // the checks away.
 #ifdef AXG_DEVICE_CHECKS
 static __device__ int32_t g_axg_check[8];  // one per translation unit
-__device__ __noinline__ bool axg_record(int kern, int line, long long idx, long long bound) {
+static __device__ __noinline__ bool axg_record(int kern, int line, long long idx, long long bound) {
   if (atomicCAS(&g_axg_check[0], 0, 1) == 0) {
     g_axg_check[1] = kern;
     g_axg_check[2] = line;
