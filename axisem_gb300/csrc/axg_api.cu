@@ -63,11 +63,6 @@ std::vector<int> axial_slots(int pole) {
   return {AXG_M0_W1, AXG_M0_W2, AXG_M0_W3, AXG_M0_W4, AXG_M0_W5, AXG_M0_W6};
 }
 
-struct DevBuf {
-  void *p = nullptr;
-  size_t n = 0;
-};
-
 // one domain of the step on the device (axg_stream.cuh)
 struct DomainDev {
   float *blocks = nullptr, *tails = nullptr;
@@ -3174,7 +3169,7 @@ constexpr int kBatchSteps = 8;
 struct axg_batch {
   std::vector<axg_handle *> hs;
   std::vector<uint8_t> streams;  // per solve: its element blocks come from HBM in a step of the batch
-  int device = 0, num_sms = 1;
+  int device = 0;
   SpecDev spec{};
   cudaStream_t stream = nullptr;
   // one step of every solve, captured with the Newmark solves' buffer roles at
@@ -3388,7 +3383,6 @@ int batch_create_impl(axg_batch *b, axg_handle *const *hs, int32_t n) {
   }
   b->device = hs[0]->device;
   b->spec = hs[0]->spec;
-  b->num_sms = hs[0]->num_sms;
   // A step of the batch reads every mesh's blocks once: where they exceed L2
   // together, also a small mesh's come from HBM, unless several solves read
   // them.  Six solves on 9 to 51 MB of blocks, 96 steps: 8.56 ms with the

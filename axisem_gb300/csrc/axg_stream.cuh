@@ -57,6 +57,7 @@ constexpr int kFluidFs = 8;
 __host__ __device__ constexpr int64_t grp_count(int64_t nel) { return (nel + kGrp - 1) / kGrp; }
 // bit 31 of a lane's first index word: axial element
 constexpr uint32_t kGrpAxial = 1u << 31, kGrpIdx = 0x0FFFFFFFu;
+static_assert(kGrpIdx == kPtIndexMask, "the planner refuses meshes of more points");
 
 // A group: its first element slot, its element count and (patched) how many
 // groups of its patch must have accumulated before it may.
@@ -773,7 +774,7 @@ __device__ __forceinline__ void solid_group(const StreamWork &w, const SpecDev &
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
       int32_t p = idx[i];
-      if (PATCH) p = p < n_int ? int_start + p : s_def[p - n_int];
+      if (PATCH) p = p < n_int ? int_start + p : AXG_BOUND(p - n_int, kMaxDef, 62) ? s_def[p - n_int] : 0;
       if (!AXG_BOUND(p, st.nglob, 62)) p = 0;
 #pragma unroll
       for (int c = 0; c < NC; ++c) u[c][i] = gather_u<MODE, KAHAN>(st, gc(c), p);
@@ -1042,7 +1043,7 @@ struct Copies {
   __device__ __forceinline__ Copies(const StreamDomain &d, uint32_t k0, uint32_t end) : k(k0), s1(end) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      e[q] = k + q < s1 ? __ldg(d.ent + k + q) : -1;
+      e[q] = k + q < s1 && AXG_BOUND(k + q, d.n_ent, 65) ? __ldg(d.ent + k + q) : -1;
       if (e[q] >= 0 && !AXG_BOUND(e[q] + FSTEP * (NC - 1), d.n_fel, 65)) e[q] = -1;
     }
   }
@@ -1058,6 +1059,7 @@ struct Copies {
 #pragma unroll
         for (int c = 0; c < NC; ++c) s[c] = s[c] + x[q][c];
     for (uint32_t q = k + 4; q < s1; ++q) {
+      if (!AXG_BOUND(q, d.n_ent, 65)) break;
       const int32_t f = __ldg(d.ent + q);
       if (!AXG_BOUND(f + FSTEP * (NC - 1), d.n_fel, 65)) break;
 #pragma unroll
@@ -1281,8 +1283,8 @@ __device__ __forceinline__ void solid_point(const StreamWork &w, int64_t g) {
 #pragma unroll
   for (int c = 0; c < NC; ++c) sum[c] = 0.f;
   if (coupled) {
-    const int32_t q = __ldg(d.ent + (s0 & kStMask));
-    if (MODE != MODE_FORCE) {
+    const int32_t q = AXG_BOUND(s0 & kStMask, d.n_ent, 66) ? __ldg(d.ent + (s0 & kStMask)) : 0;
+    if (MODE != MODE_FORCE && AXG_BOUND(q, w.to_solid.n, 66)) {
       // bdry_copy2solid (SOLVER/time_evol_wave.F90:1577-1611): b1 ddchi (s [and
       // phi]) and b2 ddchi (z) of the new fluid acceleration, formed here from
       // the fluid's contributions (with absorbing terms, stored by the launch before)
@@ -1358,7 +1360,8 @@ __device__ __forceinline__ void patch_cta(const StreamWork &w, const SpecDev &sp
   for (int t = threadIdx.x; t < n_pts; t += kGrpThreads)
 #pragma unroll
     for (int c = 0; c < NC; ++c) s.f[c][t] = 0.f;
-  for (int t = threadIdx.x; t < pi.n_def; t += kGrpThreads) s.def[t] = __ldg(d.def + pi.def_start + t);
+  for (int t = threadIdx.x; t < pi.n_def; t += kGrpThreads)
+    s.def[t] = AXG_BOUND(pi.def_start + t, d.n_def, 69) ? __ldg(d.def + pi.def_start + t) : 0;
   if (threadIdx.x == 0) s.done = 0;
   if (__syncthreads_or(gone)) return;
   // the own points' state, which the last phase reads, into L2 meanwhile
@@ -1432,7 +1435,7 @@ __device__ __forceinline__ void patch_cta(const StreamWork &w, const SpecDev &sp
     v.y = s.f[1][pi.n_int + t];
     v.z = NC == 3 ? s.f[NC - 1][pi.n_int + t] : 0.f;
     v.w = 0.f;
-    reinterpret_cast<float4 *>(d.fel)[pi.def_start + t] = v;
+    if (AXG_BOUND(4 * (pi.def_start + t) + 3, d.n_fel, 69)) reinterpret_cast<float4 *>(d.fel)[pi.def_start + t] = v;
   }
   // the patch's own points; kB at a time, their loads together
   bool src = false;
