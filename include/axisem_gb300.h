@@ -514,11 +514,12 @@ int axg_time_stiffness(axg_handle *h, int32_t n, float *ms_avg);
  * bound lo, bound hi}; returns AXG_ERR_UNSUPPORTED in normal builds. */
 int axg_device_check_report(int32_t *out8);
 
-/* Self-test of the kernels' bounded device wait: one GPU thread waits on an
- * mbarrier that nothing arrives at (no copy is involved), through the same
- * wait the patch kernels use.  *status receives what the wait recorded
- * (AXG_ERR_TIMEOUT when it gave up as designed) and *elapsed_s how long it
- * waited (about one second).  No counterpart in the reference. */
+/* Self-test of the kernels' bounded device waits: a GPU thread waits on an
+ * mbarrier that nothing arrives at (no copy is involved), as the no-allocation
+ * kernel waits, and a warp for its turn to accumulate behind a group that never
+ * does, as the patched element pass waits.  *status receives what the waits
+ * recorded (AXG_ERR_TIMEOUT when both gave up as designed) and *elapsed_s how
+ * long they took (about one second).  No counterpart in the reference. */
 int axg_selftest_wait_timeout(int32_t *status, double *elapsed_s);
 
 void axg_destroy(axg_handle *h);
