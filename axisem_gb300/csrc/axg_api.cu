@@ -942,6 +942,9 @@ cudaError_t stream_ctas(int pole, const StreamKernel &k, int *per_sm) {
 // without / with these, sphere meshes: 30 MB of blocks 12.3 / 13.1 us
 // (monopole), 36 MB 12.9 / 13.9 (quadrupole), 41 MB 16.9 / 15.8 (monopole),
 // 47 MB 17.5 / 16.4 (dipole), 51 MB 18.6 / 17.1, 64 MB 26.5 / 22.4 (dipole).
+// With cg4 attenuation, whose constants and state are not counted here, the line
+// lies there too: 30 MB 16.7 / 16.7 us (monopole), 37 MB 22.2 / 21.3, 46 MB 30.3 /
+// 25.6; 29 MB 16.7 / 16.9 (dipole), 38 MB 20.5 / 20.6, 48 MB 25.5 / 22.9.
 constexpr int64_t kL2Resident = 38 << 20;
 int64_t block_bytes(const axg_handle *h) { return h->nel_s * 100 * (n_terms(h->pole) + 1); }
 bool streamed(const axg_handle *h) { return block_bytes(h) > kL2Resident; }
@@ -954,7 +957,7 @@ StreamKernel step_kernel(const axg_handle *h, int kind) {
 
 // resident CTAs per SM of the element passes the handle's modes select
 int prepare_kernels(axg_handle *h) {
-  CK(stream_ctas(h->pole, {kElemPass, MODE_FORCE, h->os.patched, false, false, false}, &h->elem_ctas_force));
+  CK(stream_ctas(h->pole, {kElemPass, MODE_FORCE, h->os.patched, false, false, streamed(h)}, &h->elem_ctas_force));
   CK(stream_ctas(h->pole, step_kernel(h, kElemPass), &h->elem_ctas_step));
   return AXG_OK;
 }
@@ -1090,7 +1093,7 @@ void launch_anel_full(axg_handle *h, cudaStream_t s, bool update) {
 void enqueue_force(axg_handle *h, cudaStream_t s) {
   const StreamWork w = stream_work(h, MODE_FORCE, solid_state(h), StateArgs{});
   stream_launches(h, MODE_FORCE, w, [&](int kind, const StreamWork &x) {
-    launch_stream(h, {kind, MODE_FORCE, h->os.patched, false, false, false}, x, s);
+    launch_stream(h, {kind, MODE_FORCE, h->os.patched, false, false, streamed(h)}, x, s);
   });
 }
 

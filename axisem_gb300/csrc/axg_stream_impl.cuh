@@ -25,7 +25,8 @@ unsigned blocks(const StreamMany &p) { return (unsigned)p.start[p.n]; }
 // CTAs per SM of the scattered element pass.  Quadrupole steps, 4 / 3 CTAs: from
 // L2 12.9 / 14.0 us on 13 390 elements, from HBM 20.1 / 17.0 on 18 944, 23.9 /
 // 23.6 on 25 802, 32.4 / 33.2 on 32 298 (3 waves either way), 73.2 / 71.3 on
-// 70 528.  Several solves' launches, whose waves fill, keep 4: six solves on
+// 70 528.  Stiffness calls likewise: 15.9 / 13.9 us on 16 900, 53.3 / 51.3 on 62 500,
+// 103.6 / 100.1 on 129 600; dipole 14.6 / 12.7, 49.4 / 44.5, 95.5 / 86.8.  Several solves' launches, whose waves fill, keep 4: six solves on
 // 5 664 and 18 944 elements 9.67 / 9.95 ms for 96 steps.
 template <int POLE, int MODE, bool ANEL, bool KAHAN, class P>
 auto scatter_of(const StreamKernel &k) -> void (*)(P, SpecDev) {

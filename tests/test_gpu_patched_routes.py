@@ -119,3 +119,13 @@ def test_patched_solid_attenuated_at_every_point(gpu_lib, orc, pole):
 @pytest.mark.parametrize("pole", [0, 1, 2])
 def test_patched_solid_compensated_symplectic(gpu_lib, orc, pole):
     _against_oracle(orc, _mesh(PATCHED, pole, src_row=11), 4, scheme=_abi.SCHEME_SYMPLEC4, comp=True)
+
+
+@pytest.mark.parametrize("pole", [0, 1, 2])
+@pytest.mark.parametrize("size", [(60, 50, 5), (187, 151, 5)])
+def test_stiffness_call_and_step_take_the_same_form(gpu_lib, pole, size):
+    """Scattered dipoles and quadrupoles whose blocks come from HBM run at three
+    CTAs per SM, others at four, the stiffness call as the step."""
+    with Solver(_mesh(size, pole, src_row=4)) as s:
+        info = s.info()
+    assert info["ctas_per_sm_force"] == info["ctas_per_sm_step"] == (3 if pole > 0 and size[0] > 100 else 4)
