@@ -642,24 +642,40 @@ __device__ __forceinline__ void col_stiffness(const SpecDev &sp, const float (&e
     }
   }
   // second stage: f and mxm(G, S1) and mxm(S2, G2T), S1 in X, each sum formed
-  // apart and added in the reference's order.  Ten terms in a chain on top of f
-  // round at f's magnitude (stiffness errors against FP64 of 6.7e-8, these
-  // 6.3e-8, quadrupole), and f + (first + second) has 6.6e-8.  The additions
-  // cost 4 % of a quadrupole's step from HBM (19.7 to 20.6 us on 18 944 elements)
-  // and of an attenuated dipole's (131 to 136 on 99 450); others take as long.
+  // apart.  Ten terms in a chain on top of f round at f's magnitude (stiffness
+  // errors against FP64 of 6.7e-8, these 6.3e-8, quadrupole), and f + (first +
+  // second) has 6.6e-8.  The order of the two additions is the faster of each
+  // form (ms, first / second sum first): scattered quadrupole steps from HBM 4.05 /
+  // 3.75 for 200 on 18 944 elements, patched ones 21.6 / 22.0 for 32 on 786 432.
+  // (One chain takes 3.94 and 21.6, a stiffness call of 2^20 quadrupoles 0.629,
+  // with this 0.641.)
   xch_put<NC>(xw, lane, S2);
   __syncwarp();
   float Y[NC][5];
-  col_xi<NC, true>(gxi, X, Y);
-  xch_eta<NC>(xw, e5, seta, E);
+  auto local = [](int c) { return POLE == POLE_DI ? c != 0 : POLE == POLE_QUAD || c == 0; };  // f[c] has a local part
+  if (PATCH || POLE == POLE_DI) {
+    col_xi<NC, true>(gxi, X, Y);
+    xch_eta<NC>(xw, e5, seta, E);
 #pragma unroll
-  for (int c = 0; c < NC; ++c)
+    for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      if (POLE == POLE_DI ? c == 0 : POLE == POLE_MONO && c == 1) f[c][i] = Y[c][i] + E[c][i];  // (no local part)
-      else if (POLE == POLE_DI) f[c][i] = Y[c][i] + E[c][i] + f[c][i];
-      else f[c][i] = f[c][i] + Y[c][i] + E[c][i];
-    }
+      for (int i = 0; i < 5; ++i) {
+        if (!local(c)) f[c][i] = Y[c][i] + E[c][i];
+        else if (POLE == POLE_DI) f[c][i] = Y[c][i] + E[c][i] + f[c][i];
+        else f[c][i] = f[c][i] + Y[c][i] + E[c][i];
+      }
+  } else {
+    xch_eta<NC>(xw, e5, seta, E);
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int i = 0; i < 5; ++i) E[c][i] = local(c) ? f[c][i] + E[c][i] : E[c][i];
+    col_xi<NC, true>(gxi, X, Y);
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+      for (int i = 0; i < 5; ++i) f[c][i] = E[c][i] + Y[c][i];
+  }
   __syncwarp();
   if (AX) {
     auto w = [&](int q) { return m0[5 * q + j]; };
@@ -1363,7 +1379,8 @@ __device__ __forceinline__ void patch_cta(const StreamWork &w, const SpecDev &sp
   for (int t = threadIdx.x; t < pi.n_def; t += kGrpThreads)
     s.def[t] = AXG_BOUND(pi.def_start + t, d.n_def, 69) ? __ldg(d.def + pi.def_start + t) : 0;
   if (threadIdx.x == 0) s.done = 0;
-  if (__syncthreads_or(gone)) return;
+  if (MODE == MODE_FORCE) __syncthreads();
+  else if (__syncthreads_or(gone)) return;
   // the own points' state, which the last phase reads, into L2 meanwhile
   if (w.prefetch > 0 && MODE != MODE_FORCE && warp == kGrpWarps - 1 && pi.n_int > 0) {
     auto range = [&](const float *a) {
