@@ -1360,9 +1360,8 @@ int symplectic_coefficients(int scheme, std::vector<double> &cd, std::vector<dou
   return (int)cv.size();
 }
 
-// resident CTAs of the solid patch kernels on the current device (two per
-// SM), which the patch tuner spreads a colour's patches over; 0 without a
-// device
+// CTAs of the patch tuner's latency model on the current device (two per SM, as
+// the no-allocation kernel has); 0 without a device
 int solid_plan_ctas() {
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -1374,7 +1373,7 @@ int solid_plan_ctas() {
 }
 
 // tuned (or requested) patch shape, then the plan; ctas: as solid_plan_ctas
-// (0: the tuner assumes full launches); anel: the attenuated solid kernel
+// (0: the tuner assumes full launches); anel: the solid has cg4 attenuation
 std::string plan_domain(const int32_t *igloc, int64_t nel, int64_t nglob, int patch_elems, int growth,
                         const std::vector<uint8_t> &prepass, DomainPlan &plan, bool renumber = true,
                         int ctas = 0, bool anel = false) {
@@ -1826,8 +1825,8 @@ int create_impl(axg_handle *h, const axg_mesh_desc *d, const axg_handle *share =
 // Stiffness + assembly for callers that cannot allocate device memory: code
 // running where cudaMalloc is unavailable or forbidden (inside another
 // runtime's memory pool, a driver callback, a process whose device memory is
-// fully reserved up front).  It runs the same planner and the same
-// solid_patch_kernel<pole, FORCE> as axg_stiffness_assembled, but every
+// fully reserved up front).  It runs the plan of the allocating entry point
+// patch by patch and colour by colour (solid_patch_kernel<pole>), and every
 // device-side buffer -- plan, packed element blocks, u, f and control words --
 // lives in one file-scope static device array of kNoAllocScratchBytes.  Each
 // GPU that loads this library holds that array until the process exits.
@@ -2086,7 +2085,7 @@ int anel_state_io(axg_handle *h, int field, float *out, const float *in) {
 
 extern "C" {
 
-const char *axg_version(void) { return "axisem_gb300 1 (sm_103a, patch-coloured assembly)"; }
+const char *axg_version(void) { return "axisem_gb300 1 (sm_103a, element pass and point pass)"; }
 
 int axg_device_count(void) {
   int n = 0;
@@ -2205,8 +2204,8 @@ int axg_run(axg_handle *h, int32_t first_iter, int32_t n_iter) {
   CK(cudaMemcpyAsync(h->ctl + CTL_ITER, &first_iter, sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
   CK(refresh_predicted(h, h->stream));
   // Graph q + 1 is queued before the flags of graph q are waited for, so that
-  // the device does not idle while the host polls (a stopped solve's kernels
-  // return at once).  Polling each graph before the next had cost 10 us per
+  // the device does not idle while the host polls (a stopped solve's steps do
+  // nothing).  Polling each graph before the next had cost 10 us per
   // graph: 3.66 against 3.40 ms for 400 steps of the PREM 50 s mesh.
   auto poll = [&](int q) -> int {
     CK(cudaEventSynchronize(h->ev_flags[q & 1]));
@@ -2480,8 +2479,8 @@ int axg_run_async(axg_handle *h, int32_t first_iter, int32_t n_iter) {
       return fail(h, AXG_ERR_BAD_ARG, fmt("snapshot %lld of the run is beyond the dump buffer's capacity %lld",
                                           (long long)last, (long long)dp.capacity));
   }
-  // the kernels of a step after a blow-up return at once, so all steps can
-  // be queued without a check in between
+  // the steps after a blow-up do nothing, so all steps can be queued without a
+  // check in between
   CK(cudaMemcpyAsync(h->ctl + CTL_ITER, &first_iter, sizeof(int32_t), cudaMemcpyHostToDevice, h->stream));
   CK(refresh_predicted(h, h->stream));
   for (int32_t done = 0; done < n_iter;) {

@@ -153,7 +153,7 @@ struct StateArgs {
 
 // A launch's per-solve arguments, passed in its parameter space
 // (__grid_constant__).  One<W>: one solve owns all of the launch's work items
-// (a colour's patches, the boundary points, ...).  Many<W>: up to kMaxBatch
+// (its points, its receivers).  Many<W>: up to kMaxBatch
 // solves advanced together by one launch; solve s owns the items
 // [start[s], start[s + 1]), and a CTA or thread finds its solve from them.
 constexpr int kMaxBatch = 32;

@@ -106,6 +106,12 @@ int64_t plan_latency(const DomainPlan &plan, int ctas, int overhead);
 // plan_latency of the whole mesh over sizes down to 8 elements: a colour is
 // about one round of patches, and smaller patches spread it over more CTAs.
 // patch_elems > 0 or growth >= 0 fix that choice.
+// Both models are of colours launched one after another, as the no-allocation
+// stiffness runs them.  The step has no colours.  In a scattered solid the shape
+// decides the order of elements alone (PREM 50 s, patches of 8 / 64 elements: 9.80
+// / 9.83 us per step; 25 s, 24 / 64: 19.7 / 19.9); a patched solid of 131 406
+// elements, the one size range where the models differ, takes 118.1 us with the
+// 56 they choose and 120.4 with 64 (quadrupole; monopole 76.8 / 80.5).
 constexpr int kTuneFullRounds = 2;
 std::string tune_plan(const int32_t *igloc, int64_t nel, int64_t nglob, int patch_elems, int growth,
                       int *best_pe, int *best_growth, int ctas = 0, int overhead = kPatchOverheadElastic);

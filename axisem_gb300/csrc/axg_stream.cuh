@@ -21,8 +21,12 @@
 // the xi contractions are in-lane FMAs with constant-bank matrices, and the
 // eta contractions read the other columns from a per-warp shared buffer as
 // broadcast 16-byte loads: 4 stores and 20 loads per warp and stage for six
-// elements, where a lane per point takes 30 shuffles per element.  About 150
-// warp instructions per element against about 380.
+// elements, where a lane per point takes 30 shuffles per element.  Warp
+// instructions counted per solid element (with a fifth to a third as many fluid
+// elements): 193 scattered quadrupole, 320 dipole with cg4 attenuation, 337 patched
+// quadrupole and 248 monopole, which finish points as well; a lane per point took
+// 380 without those.  Issue slots are 24 to 40 % used: what bounds the pass from
+// HBM is the loads in flight of 11 to 16 resident warps per SM.
 //
 // Element arrays are packed per group of up to six consecutive element slots,
 // in rows of eight floats per lane (one 256-bit load each): a lane's values
@@ -1101,8 +1105,9 @@ struct FluidForce {
   }
 };
 
-// One fluid point: the corrector as fluid_point_kernel's; a Newmark step
-// stores the next prediction (the compensated one with the compensation it
+// One fluid point: ddchi = -inv_mass_fluid * force [- absorbing terms], dchi by
+// the Newmark corrector or a symplectic kick, chi (zero on the axis for the
+// non-monopole sources); a Newmark step stores the next prediction (the compensated one with the compensation it
 // leaves, cup).
 template <bool NONMONO, int MODE, bool KAHAN>
 __device__ __forceinline__ void fluid_point(const StreamWork &w, int64_t g) {
