@@ -284,6 +284,17 @@ __device__ __forceinline__ void col_xi(const float *g, const float (&v)[NC][5], 
     }
 }
 
+// out[c][i] += sum_k g[i + 5 k] v[c][k], term by term
+template <int NC>
+__device__ __forceinline__ void col_xi_add(const float *g, const float (&v)[NC][5], float (&out)[NC][5]) {
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+#pragma unroll
+      for (int k = 0; k < 5; ++k) out[c][i] = fmaf(g[i + 5 * k], v[c][k], out[c][i]);
+}
+
 // component c of a group array is the axis-masked one of the pole (group
 // arrays hold s, z for the monopole)
 template <int POLE>
@@ -645,19 +656,21 @@ __device__ __forceinline__ void col_stiffness(const SpecDev &sp, const float (&e
       }
     }
   }
-  // second stage: f and mxm(G, S1) and mxm(S2, G2T), S1 in X, each sum formed
-  // apart.  Ten terms in a chain on top of f round at f's magnitude (stiffness
-  // errors against FP64 of 6.7e-8, these 6.3e-8, quadrupole), and f + (first +
-  // second) has 6.6e-8.  The order of the two additions is the faster of each
-  // form (ms, first / second sum first): scattered quadrupole steps from HBM 4.05 /
-  // 3.75 for 200 on 18 944 elements, patched ones 21.6 / 22.0 for 32 on 786 432.
-  // (One chain takes 3.94 and 21.6, a stiffness call of 2^20 quadrupoles 0.629,
-  // with this 0.641.)
+  // second stage: f and mxm(G, S1) and mxm(S2, G2T), S1 in X.  All ten terms in a
+  // chain on top of f round at f's magnitude; the second sum at least is formed
+  // apart.  Stiffness errors against FP64, 1e-8, quadrupole, random metric terms /
+  // PREM mesh: chain 8.58 / 7.43, both sums apart as the reference adds them 8.23 /
+  // 6.90, the second one apart 8.16 / 6.61.  The last is the faster one for a
+  // scattered quadrupole's or monopole's pass (200 compensated steps of 18 944
+  // elements: 3.97, 4.05 and 3.83 ms); patched, attenuated and dipole passes are as
+  // fast or faster with both apart (32 steps of 786 432 elements 21.7 ms, 72 of
+  // 99 450 attenuated 9.4, where the last takes 9.8).  A stiffness call of 2^20
+  // quadrupoles took 0.629 ms with the chain and takes 0.641.
   xch_put<NC>(xw, lane, S2);
   __syncwarp();
   float Y[NC][5];
   auto local = [](int c) { return POLE == POLE_DI ? c != 0 : POLE == POLE_QUAD || c == 0; };  // f[c] has a local part
-  if (PATCH || POLE == POLE_DI) {
+  if (PATCH || ANEL || POLE == POLE_DI) {
     col_xi<NC, true>(gxi, X, Y);
     xch_eta<NC>(xw, e5, seta, E);
 #pragma unroll
@@ -669,16 +682,12 @@ __device__ __forceinline__ void col_stiffness(const SpecDev &sp, const float (&e
         else f[c][i] = f[c][i] + Y[c][i] + E[c][i];
       }
   } else {
+    col_xi_add<NC>(gxi, X, f);
     xch_eta<NC>(xw, e5, seta, E);
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
-      for (int i = 0; i < 5; ++i) E[c][i] = local(c) ? f[c][i] + E[c][i] : E[c][i];
-    col_xi<NC, true>(gxi, X, Y);
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int i = 0; i < 5; ++i) f[c][i] = E[c][i] + Y[c][i];
+      for (int i = 0; i < 5; ++i) f[c][i] = f[c][i] + E[c][i];
   }
   __syncwarp();
   if (AX) {
